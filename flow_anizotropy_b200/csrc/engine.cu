@@ -272,7 +272,7 @@ static void lbm_group_items(std::vector<Solve3> &hs, std::vector<int2> &items)
 
 cudaError_t lbm_launch_step(int prec, int variant, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a)
 {
-    if (prec == LBM_FP64) return launch_step3d_f64(variant, odd, grid, s, a);
+    if (prec == LBM_FP64) return launch_step3d_f64(variant, w1, odd, grid, s, a);
     if (is_dense_m(prec)) return launch_stepmd(variant, grid, s, a);
     if (is_moment(prec)) return launch_stepm(prec, variant, grid, s, a);
     return launch_step3d_lp(prec, variant, w1, odd, grid, s, a);
@@ -316,6 +316,21 @@ void lbm_fill_solve3(Solve3 &S, int nx, int ny, int nz, const double F[3], const
     for (int c = 0; c < 3; ++c) { P.F[c] = F[c]; P.Ff[c] = (float)F[c]; }
     P.tau = p.tau;
     P.pref = 1.0 - 0.5 / p.tau;
+    P.itau = 1.0 / p.tau;
+    P.wp[0] = w3(0) * P.pref; P.wp[1] = w3(1) * P.pref; P.wp[2] = w3(7) * P.pref;
+    for (int j = 0; j < 9; ++j) {
+        // zero products dropped, as the collision's (x + 0 == x)
+        const int k = 2 * j + 1, e[3] = {ex3(k), ey3(k), ez3(k)};
+        double eF = 0.0;
+        bool first = true;
+        for (int c = 0; c < 3; ++c) {
+            if (!e[c]) continue;
+            const double t = e[c] > 0 ? F[c] : -F[c];
+            eF = first ? t : eF + t;
+            first = false;
+        }
+        P.eF[j] = eF;
+    }
     P.omega = (float)(1.0 / p.tau);
     P.preff = (float)P.pref;
     // FP16 keeps h * scale; scale puts the largest plausible deviation

@@ -652,7 +652,7 @@ template <class ST, bool W1, class Cp>
 __device__ __forceinline__ void collide3(Cp (&g)[Q3], const Solve3 &S, Cp &ux, Cp &uy, Cp &uz)
 {
     if constexpr (ST::shifted) collide_pairs<W1, F32x1>(g, S.P, S.scale, S.inv_scale, ux, uy, uz);
-    else collide_ref64(g, S.P, ux, uy, uz);
+    else collide_ref64<W1>(g, S.P, ux, uy, uz);
 }
 
 // Two voxels' populations collided together (packed FP32, the same bits per
@@ -816,7 +816,7 @@ struct BulkTile {
     unsigned tile_start;     // rank of the tile's first voxel
     unsigned P, nfluid;
     float scale, inv_scale;
-    Phys3 phys;
+    PhysF phys;
 };
 
 // Odd (local) step staged through shared memory by the copy engine.  A
@@ -1017,7 +1017,7 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
 #pragma unroll
         for (int k = 0; k < Q3; ++k) ST::lds2(buf + (k * TV + 2u * tid), g[k].x, g[k].y);
         const float sc = d.scale, isc = d.inv_scale;
-        const Phys3 phys = d.phys;
+        const PhysF phys = d.phys;
         const int solve = d.solve;
         const unsigned tstart = d.tile_start;
         mbar_arrive(&empty[s]);    // this thread is done with buffer s (and its descriptor)
@@ -1793,7 +1793,7 @@ __global__ void canon3d_kernel(const Solve3 S, long long done, double *f_out, fl
 // contraction to keep the reference's rounding).
 // `odd`: launch the odd-step (local) kernel, else the even-step one; every
 // solve in the launch must be at a step of that parity.
-cudaError_t launch_step3d_f64(int variant, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a);
+cudaError_t launch_step3d_f64(int variant, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a);
 cudaError_t launch_step3d_lp(int prec, int variant, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a);
 cudaError_t launch_init3d(int prec, void *A, long long plane, long long n, cudaStream_t s);
 // Allow the bulk-staged odd kernels their shared-memory ring on device `dev`

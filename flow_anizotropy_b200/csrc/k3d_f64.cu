@@ -5,14 +5,12 @@
 
 namespace lbm {
 
-#define LBM_ODD(V) step3d_odd_kernel<StoreF64, odd_f64(V).npt, odd_f64(V).minb, false>
-#define LBM_EVEN(V) step3d_even_kernel<StoreF64, even_f64(V).minb, false, even_meta(V)>
+#define LBM_ODD(V) step3d_odd_kernel<StoreF64, odd_f64(V).npt, odd_f64(V).minb, W1>
+#define LBM_EVEN(V) step3d_even_kernel<StoreF64, even_f64(V).minb, W1, even_meta(V)>
 
-cudaError_t launch_step3d_f64(int variant, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a)
+template <bool W1>
+static void launch_f64(int vo, int ve, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a)
 {
-    if (variant < 0 || variant >= 2 * NVAR_F64) return cudaErrorInvalidValue;
-    variant = kernel_variant(0, variant);        // the two-lattice AA form runs the in-place kernels
-    const int vo = variant / NVAR_EVEN, ve = variant % NVAR_EVEN;
     if (odd) {
         switch (vo) {
         case 0: LBM_ODD(0)<<<grid, TPB, 0, s>>>(a); break;
@@ -31,11 +29,21 @@ cudaError_t launch_step3d_f64(int variant, bool odd, dim3 grid, cudaStream_t s, 
         default: LBM_EVEN(1)<<<grid, TPB, 0, s>>>(a); break;
         }
     }
+}
+
+cudaError_t launch_step3d_f64(int variant, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a)
+{
+    if (variant < 0 || variant >= 2 * NVAR_F64) return cudaErrorInvalidValue;
+    variant = kernel_variant(0, variant);        // the two-lattice AA form runs the in-place kernels
+    const int vo = variant / NVAR_EVEN, ve = variant % NVAR_EVEN;
+    if (w1) launch_f64<true>(vo, ve, odd, grid, s, a);
+    else launch_f64<false>(vo, ve, odd, grid, s, a);
     return cudaGetLastError();
 }
 
 int max_blocks_f64(int variant, bool odd)
 {
+    constexpr bool W1 = true;
     variant = kernel_variant(0, variant);
     const int vo = variant / NVAR_EVEN, ve = variant % NVAR_EVEN;
     const void *k = odd ? (vo == 0 ? (const void *)LBM_ODD(0) : vo == 1 ? (const void *)LBM_ODD(1) : (const void *)LBM_ODD(2))
