@@ -365,12 +365,17 @@ struct StoreF16 {
         lo = __half2float(__ushort_as_half((unsigned short)(w & 0xffffu)));
         hi = __half2float(__ushort_as_half((unsigned short)(w >> 16)));
     }
-    __device__ static __forceinline__ void st2(T *p, C lo, C hi, uint32_t rlo, uint32_t rhi)
+    // the two rounded halves, lo in the low one
+    __device__ static __forceinline__ uint32_t sr2(C lo, C hi, uint32_t rlo, uint32_t rhi)
     {
         const uint32_t rb = __byte_perm(rlo, rhi, 0x7632);   // high halves: rhi above, rlo below
         uint32_t d;
         asm("cvt.rs.f16x2.f32 %0, %1, %2, %3;" : "=r"(d) : "f"(hi), "f"(lo), "r"(rb));
-        __stcs(reinterpret_cast<unsigned int *>(p), d);
+        return d;
+    }
+    __device__ static __forceinline__ void st2(T *p, C lo, C hi, uint32_t rlo, uint32_t rhi)
+    {
+        __stcs(reinterpret_cast<unsigned int *>(p), sr2(lo, hi, rlo, rhi));
     }
     __host__ __device__ static constexpr double init(int) { return 0.0; }
 };
@@ -408,12 +413,17 @@ struct StoreBF16 {
         lo = __bfloat162float(__ushort_as_bfloat16((unsigned short)(w & 0xffffu)));
         hi = __bfloat162float(__ushort_as_bfloat16((unsigned short)(w >> 16)));
     }
-    __device__ static __forceinline__ void st2(T *p, C lo, C hi, uint32_t rlo, uint32_t rhi)
+    // the two rounded halves, lo in the low one
+    __device__ static __forceinline__ uint32_t sr2(C lo, C hi, uint32_t rlo, uint32_t rhi)
     {
         const uint32_t rb = __byte_perm(rlo, rhi, 0x7632);   // high halves: rhi above, rlo below
         uint32_t d;
         asm("cvt.rs.bf16x2.f32 %0, %1, %2, %3;" : "=r"(d) : "f"(hi), "f"(lo), "r"(rb));
-        __stcs(reinterpret_cast<unsigned int *>(p), d);
+        return d;
+    }
+    __device__ static __forceinline__ void st2(T *p, C lo, C hi, uint32_t rlo, uint32_t rhi)
+    {
+        __stcs(reinterpret_cast<unsigned int *>(p), sr2(lo, hi, rlo, rhi));
     }
     __host__ __device__ static constexpr double init(int) { return 0.0; }
 };

@@ -16,6 +16,7 @@
 #include "engine_host.h"
 #include "engine_m.cuh"
 #include "engine_md.cuh"
+#include "step3d_slots.cuh"
 
 using namespace lbm;
 
@@ -353,7 +354,7 @@ void lbm_fill_solve3(Solve3 &S, int nx, int ny, int nz, const double F[3], const
     c.sample = p.sample > 0 ? p.sample : 1; c.ksigma = p.ksigma;
 }
 
-void lbm_init_state3(State3 &st, const Ctl3 &c)
+void lbm_init_state3(State3 &st, const Ctl3 &c, int mode)
 {
     memset(&st, 0, sizeof(st));
     st.phase = PH_RUN;
@@ -363,6 +364,9 @@ void lbm_init_state3(State3 &st, const Ctl3 &c)
         if (c.avg_steps <= 0) { st.phase = PH_DONE; st.steps = 0; }
         else { st.phase = PH_AVG; st.avg_start = 0; }
     }
+    // reductions of the first pass (the controller pass notes the later ones)
+    for (int r = 0; r < DEFER_SLOTS; ++r)
+        if (deferred_reduces(c, st.phase, r + 1, 0, mode)) st.redm |= 1ull << r;
 }
 
 int lbm_pick_npt(const lbm_params3d &p) { return variant_npt(p.precision, p.variant); }
@@ -450,9 +454,56 @@ constexpr int kGraphSteps3 = 64;
 // size).
 bool lbm_defers(int prec) { return !is_dense_m(prec); }
 
-long long lbm_partial_doubles(int prec, int ntiles)
+long long lbm_partial_doubles(int prec, int ntiles, bool split)
 {
-    return 3ll * ntiles * (lbm_defers(prec) ? DEFER_SLOTS : 1);
+    return 3ll * ntiles * (lbm_defers(prec) ? DEFER_SLOTS : 1) * (split ? TPB / 32 : 1);
+}
+
+// Do solves of this (effective) variant run the kernels of step3d_slots.cuh?
+// The default variants do, and their one- and two-lattice counterparts: FP64
+// variants 0 and 18, the pull form with ranks from the record, the bulk-staged
+// odd + link-slot even pair (69 in place, 150).  The others, and structures
+// without neighbour records (whose effective variant computes ranks), run the
+// work-list kernels of engine3d.cuh.
+bool lbm_slots_variant(int prec, int variant)
+{
+    if (prec == LBM_FP64) return kernel_variant(prec, variant) == 0;
+    if (prec > LBM_BF16) return false;
+    return variant == NVAR_LP + 1 || kernel_variant(prec, variant) == 4 * NVAR_EVEN_LP + 9;
+}
+
+// Are the tiles of a single solve split over several blocks (Solve3::split)?
+// Up to SPLIT_MAX_TILES tiles in all of a call's directions: 100 MB of
+// partials at most, and beyond it the last wave of whole tiles is a small
+// part of a step.  The pull form's whole tiles pack better (its split tiles
+// measured the same at 96^3, 42.5 against 42.6 us per step), so it splits
+// only where whole tiles do not fill the SMs' block slots once.
+constexpr int SPLIT_MAX_TILES = 8192, SPLIT_MAX_TILES_PULL = 444;
+static bool plain_split(int prec, int variant, const Solve3 &S, int ndir)
+{
+    variant = lbm_effective_variant(prec, variant, S.meta != nullptr);
+    return lbm_slots_variant(prec, variant) &&
+           (long long)S.ntiles * ndir <= (is_pull_variant(prec, variant) ? SPLIT_MAX_TILES_PULL : SPLIT_MAX_TILES);
+}
+
+// One step of the plain solves hs by the kernels of step3d_slots.cuh.
+static cudaError_t launch_plain_slots(const std::vector<Solve3> &hs, int prec, int variant, bool w1, const StepArgs &a, cudaStream_t s)
+{
+    const bool pull = is_pull_variant(prec, variant);
+    // directions per launch: a structure's group where the even step is
+    // grouped, else as many as the parameters hold
+    const int n = (int)hs.size(), per = lbm_grouped_variant(prec, variant) ? MAX_GROUP : MAX_PLAIN;
+    cudaError_t e = cudaSuccess;
+    for (int j = 0; j < n && e == cudaSuccess; j += per) {
+        SlotArgs<false> x;
+        const int m = std::min(per, n - j);
+        for (int d = 0; d < m; ++d) x.s[d] = hs[j + d];
+        x.a = a;
+        const bool odd = a.n4 & 1;
+        e = prec == LBM_FP64 ? launch_slots3d_f64(w1, odd, hs[j].split, hs[j].ntiles, m, s, x)
+                             : launch_slots3d_lp(prec, pull, w1, odd, hs[j].split, hs[j].ntiles, m, s, x);
+    }
+    return e;
 }
 
 static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, State3 *d_states,
@@ -494,7 +545,14 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
     ae.wait_ns = a.wait_ns;
     ae.starve = a.starve;
     const bool gall = lbm_grouped_all(prec, variant);
-    auto launch = [&](long long rel, bool odd) {
+    const bool slots = lbm_slots_variant(prec, variant);
+    auto launch = [&](long long rel, int n4, int bit) {
+        const bool odd = n4 & 1;
+        if (slots) {
+            StepArgs x = a;
+            x.step = rel; x.bit = bit; x.n4 = n4;
+            return launch_plain_slots(hs, prec, variant, w1, x, ctx->stream);
+        }
         StepArgs x = (odd && !gall) ? a : ae;
         x.step = rel;
         return lbm_launch_step(prec, variant, w1, odd, dim3(x.nwork), ctx->stream, x);
@@ -503,7 +561,7 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
     // before a chunk reuses their slots, and before the states are read)
     auto flush = [&]() -> cudaError_t {
         if (!pending) return cudaSuccess;
-        const cudaError_t e = launch_deferred3d(d_solves, n, pend0, pending, qb, 1, ctx->stream);
+        const cudaError_t e = launch_deferred3d(d_solves, n, pend0, pending, qb, 1, 0, ctx->stream);
         pending = 0;
         return e;
     };
@@ -526,10 +584,10 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
         if (!exec && target - s >= 2 * kGraphSteps3) {
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = cudaSuccess;
-            // launch i of a chunk runs step i + 1 after s_base (s_base even)
-            for (int i = 0; i < kGraphSteps3 && e == cudaSuccess; ++i) e = launch(i, ((i + 1) & 1) == 1);
-            if (e == cudaSuccess && defer) e = launch_deferred3d(d_solves, n, 0, kGraphSteps3, qb, 1, ctx->stream);
-            if (e == cudaSuccess) {
+            // launch i of a chunk runs step i + 1 after s_base (a multiple of 4)
+            for (int i = 0; i < kGraphSteps3 && e == cudaSuccess; ++i) e = launch(i, (i + 1) & 3, i);
+            if (e == cudaSuccess && defer) e = launch_deferred3d(d_solves, n, 0, kGraphSteps3, qb, 1, kGraphSteps3, ctx->stream);
+            if (e == cudaSuccess && !defer) {
                 advance3d_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(d_solves, n, kGraphSteps3);
                 e = cudaGetLastError();
             }
@@ -539,7 +597,7 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
             CK(cudaGraphInstantiate(&exec, graph, 0));
         }
         while (s < target) {
-            if (exec && (s & 1) == 0 && target - s >= kGraphSteps3) {
+            if (exec && (s & 3) == 0 && target - s >= kGraphSteps3) {
                 CK(flush());
                 if (base != s) {
                     // a chunk numbers its steps from s_base: catch up with the single steps
@@ -552,7 +610,7 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
                 base += kGraphSteps3;
             } else {
                 // every unfinished solve of the call is at step s + 1 (they start together)
-                CK(launch(s - base, ((s + 1) & 1) == 1));
+                CK(launch(s - base, (int)((s + 1) & 3), pending));
                 if (defer) {
                     if (!pending) pend0 = s - base;
                     if (++pending == DEFER_SLOTS) CK(flush());
@@ -605,13 +663,14 @@ extern "C" int lbm_solve3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, i
         lbm_copy_pores(S, proto);
         lat.emplace_back(ctx->stream);
         part.emplace_back(ctx->stream);
+        S.split = plain_split(prec, p.variant, S, ndir) ? 1 : 0;
         CK(lat.back().alloc((size_t)lbm_lattice_bytes(S)));
-        CK(part.back().alloc(sizeof(double) * (size_t)lbm_partial_doubles(prec, S.ntiles)));
+        CK(part.back().alloc(sizeof(double) * (size_t)lbm_partial_doubles(prec, S.ntiles, S.split)));
         lbm_attach_lattice(S, lat.back().p);
         S.mask = static_cast<const uint32_t *>(mask.p);
         S.partials = static_cast<double *>(part.back().p);
         S.st = static_cast<State3 *>(d_states.p) + j;
-        lbm_init_state3(hst[j], S.c);
+        lbm_init_state3(hst[j], S.c, 1);
         CK(lbm_init_lattice(prec, S, ctx->stream));
     }
     std::vector<int2> work;
@@ -706,12 +765,13 @@ extern "C" int lbm_debug_steps3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int
     rc = lbm_build_pores(ctx, S, npt, wpre, fnode, meta, meta2);
     if (rc) return rc;
     CK(lat.alloc((size_t)lbm_lattice_bytes(S)));
-    CK(part.alloc(sizeof(double) * (size_t)lbm_partial_doubles(precision, S.ntiles)));
+    S.split = plain_split(precision, variant, S, 1) ? 1 : 0;
+    CK(part.alloc(sizeof(double) * (size_t)lbm_partial_doubles(precision, S.ntiles, S.split)));
     CK(d_states.alloc(sizeof(State3)));
     lbm_attach_lattice(S, lat.p);
     S.mask = static_cast<const uint32_t *>(mask.p);
     S.partials = static_cast<double *>(part.p); S.st = static_cast<State3 *>(d_states.p);
-    lbm_init_state3(hst[0], S.c);
+    lbm_init_state3(hst[0], S.c, 1);
     CK(lbm_init_lattice(precision, S, ctx->stream));
     std::vector<int2> work;
     for (int t = 0; t < S.ntiles; ++t) work.push_back(make_int2(0, t));
@@ -812,11 +872,12 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
             F[j % 3] = 1e-6;
             lbm_fill_solve3(hs[j], nx, ny, nz, F, p, npt);
             lbm_copy_pores(hs[j], proto);
+            hs[j].split = plain_split(precision, v, hs[j], ndir) ? 1 : 0;
             lbm_attach_lattice(hs[j], lat[j].p);
             hs[j].mask = proto.mask;
             hs[j].partials = static_cast<double *>(part.p) + 3ll * j * max_tiles;
             hs[j].st = static_cast<State3 *>(d_states.p) + j;
-            lbm_init_state3(hst[j], hs[j].c);
+            lbm_init_state3(hst[j], hs[j].c, 1);
             CK(lbm_init_lattice(precision, hs[j], ctx->stream));
             for (int t = 0; t < hs[j].ntiles; ++t) work.push_back(make_int2(j, t));
         }
@@ -830,7 +891,9 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
         a.work = static_cast<const int2 *>(w.p);
         a.nwork_dev = nullptr;
         a.nwork = (int)work.size();
+        if (lbm_defers(precision)) { a.defer = 1; a.bit = 0; }      // no step reduces (redm = 0)
         const int ev = lbm_effective_variant(precision, v, proto.meta != nullptr);
+        const bool slots = lbm_slots_variant(precision, ev);
         StepArgs ae = a;
         DevMem gw(ctx->stream);
         if (lbm_grouped_variant(precision, ev)) {
@@ -847,6 +910,10 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
             const bool odd = ((s + 1) & 1) == 1;
             StepArgs &x = (odd && !gall) ? a : ae;
             x.step = s;
+            if (slots) {
+                x.n4 = (int)((s + 1) & 3);
+                return launch_plain_slots(hs, precision, ev, true, x, ctx->stream);
+            }
             return lbm_launch_step(precision, ev, true, odd, dim3(x.nwork), ctx->stream, x);
         };
         long long s = 0;

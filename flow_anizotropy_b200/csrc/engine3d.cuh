@@ -84,6 +84,7 @@ constexpr unsigned long long WAIT_NS = 1000000000ull;
 // Mutable per-solve state, device resident, written only by the controller.
 struct State3 {
     long long s_base;     // steps completed before the current launch chunk
+    unsigned long long redm;   // deferred reduction: bit r set if step r of the pass after the last controller pass reduces
     int phase;
     int hold, have_prev;
     int converged, status;
@@ -134,6 +135,7 @@ struct Solve3 {
     MDGeom md;            // dense moment form only
     int group;            // grouped even step: directions in the group led by this record (else 0)
     int pull;             // two-lattice pull form (step3d_pull_kernel): A and B alternate
+    int split;            // flux partials per warp of a tile (step3d_slots.cuh), else per tile
     int aa2;              // two-lattice AA form: the even step scatters into the other lattice (aa_buf)
 };
 
@@ -146,7 +148,41 @@ struct StepArgs {
     unsigned long long wait_ns = 0;   // bulk-staged kernels: wait limit (0: WAIT_NS)
     int starve = 0;                   // test only: the bulk producer issues nothing
     int defer = 0;                    // flux partials to deferred slots (see finish_tile)
+    int bit = -1;                     // deferred: bit of State3::redm that says whether this step reduces
+    int n4 = -1;                      // step number modulo 4, where all solves of the launch share it
 };
+
+// Solve records of one launch of a single solve; calls with more directions
+// take several launches per step.
+constexpr int MAX_PLAIN = 4;
+template <bool LIST> struct SlotArgs;
+template <> struct SlotArgs<true> { StepArgs a; };
+template <> struct SlotArgs<false> { StepArgs a; Solve3 s[MAX_PLAIN]; };
+
+// Programmatic dependent launch: let the next grid's blocks start; wait until
+// every grid before this one has ended and its writes are visible.  Every
+// block waits before it reads what a step writes or returns, so the end of a
+// grid implies the end of all before it.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch with programmatic stream serialisation (a launch in a captured
+// stream becomes a programmatic edge of the graph).
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block, unsigned smem, cudaStream_t s, const A &...a)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
+}
 
 // Deferred reduction: with StepArgs::defer set, a reduction step leaves each
 // tile's flux partial in slot (step & (DEFER_SLOTS - 1)) of the solve's
@@ -188,7 +224,7 @@ __device__ __forceinline__ int mbit(const uint32_t *row, int x)
     return (int)((__ldg(row + (x >> 5)) >> (x & 31)) & 1u);
 }
 
-__device__ __forceinline__ bool needs_reduction(const Ctl3 &c, int phase, long long n)
+__host__ __device__ __forceinline__ bool needs_reduction(const Ctl3 &c, int phase, long long n)
 {
     if (phase == PH_AVG) return true;
     if (n == c.max_steps) return true;
@@ -339,6 +375,27 @@ __device__ __forceinline__ void block_sum3(double (&v)[3], double (*sh)[3])
     if constexpr (TRAIL) cta_sync<NT, BAR>();
 }
 
+// Sums of three values over a warp, written to out[0..2]: the shuffle tree of
+// block_sum3 (lane l takes l + 16, then l + 8, ...) with the three trees side
+// by side.  A level's sums fill half the lanes, so the other half carries
+// another component (a sum's two terms may come in either order: the same
+// bits): 6 exchanges and additions instead of 15.
+__device__ __forceinline__ void warp_sum3(const double (&v)[3], double *out)
+{
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 16, z = lane & 8;
+    // lanes 0-15: x; 16-31: y; both: z
+    const double xy = (hi ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[1], 16);
+    const double zz = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
+    // lanes 0-7: x; 8-15: z; 16-23: y
+    double s = (z ? zz : xy) + __shfl_xor_sync(0xffffffffu, z ? xy : zz, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[0] = s;
+    if (lane == 16) out[1] = s;
+    if (lane == 8) out[2] = s;
+}
+
 __device__ __forceinline__ int defer_slot(const StepArgs &a)
 {
     return a.defer ? (int)(a.step & (DEFER_SLOTS - 1)) : -1;
@@ -351,7 +408,7 @@ __device__ __forceinline__ int defer_slot(const StepArgs &a)
 // solves sit at different step counts), every step after a lag multiple or
 // max_steps since the pass started: the controller may have left phase 1
 // there and then needs every step.
-__device__ __forceinline__ bool deferred_reduces(const Ctl3 &c, int phase, long long n, long long pass_start, int mode)
+__host__ __device__ __forceinline__ bool deferred_reduces(const Ctl3 &c, int phase, long long n, long long pass_start, int mode)
 {
     if (needs_reduction(c, phase, n)) return true;
     if (mode != 2 || phase != PH_RUN) return false;
@@ -377,6 +434,11 @@ __device__ __forceinline__ void finish_tile(const Solve3 &S, int tile, long long
                                             double (&acc)[3], double (*sh)[3], int slot = -1)
 {
     __shared__ int s_last;
+    if (slot >= 0 && S.split) {            // split tiles: the warps' sums, added by reduce3d_kernel (no barrier
+                                           // here: the bulk-staged kernel has one before each tile)
+        warp_sum3(acc, S.partials + 3ll * (((long long)slot * S.ntiles + tile) * (TPB / 32) + (threadIdx.x >> 5)));
+        return;
+    }
     if (slot >= 0) {
         block_sum3<NT, BAR, true>(acc, sh);
         if (threadIdx.x == 0) {
@@ -842,9 +904,10 @@ __host__ __device__ constexpr unsigned odd_bulk_smem()
     return (unsigned)odd_bulk_stages<T>() * Q3 * TPB * TILE_NPT * (unsigned)sizeof(T);
 }
 
-template <class ST, int MINB, bool W1>
-__global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel(const StepArgs a)
+template <class ST, int MINB, bool W1, bool LIST>
+__global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel(const __grid_constant__ SlotArgs<LIST> ka)
 {
+    const StepArgs &a = ka.a;
     using T = typename ST::T;
     static_assert(TILE_NPT == 2, "a tile is one voxel pair per thread");
     constexpr int NS = odd_bulk_stages<T>();
@@ -856,8 +919,17 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
     __shared__ BulkTile slot[NS];
     __shared__ double sh[TPB / 32][3];
     __shared__ float su[3][TPB * TILE_NPT];
-    const int nwork = a.nwork_dev ? *a.nwork_dev : a.nwork;
+    pdl_launch();
+    const int nwork = (LIST && a.nwork_dev) ? *a.nwork_dev : a.nwork;
     const int tid = threadIdx.x;
+    // the solve records, and item w of the launch: (solve, tile); without a
+    // list the items are the tiles of the first solve, then of the next, ...
+    const Solve3 *solves;
+    if constexpr (LIST) solves = a.solves; else solves = ka.s;
+    auto item_of = [&](int w) {
+        if constexpr (LIST) return a.work[w];
+        else { const int nt = ka.s[0].ntiles; return make_int2(w / nt, w % nt); }
+    };
     const unsigned long long wait_ns = a.wait_ns ? a.wait_ns : WAIT_NS;
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) {
@@ -868,6 +940,7 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
         mbar_init_fence();
     }
     __syncthreads();
+    pdl_wait();
 
     if (tid >= TPB) {
         // ------------------------------------------------------ producer --
@@ -901,9 +974,9 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
                     int w = next;
                     BulkTile &d = slot[s];
                     for (; w < nwork; w += gridDim.x) {
-                        const int2 it = a.work[w];
+                        const int2 it = item_of(w);
                         if (it.x != cx) {
-                            const Solve3 &S = a.solves[it.x];
+                            const Solve3 &S = solves[it.x];
                             cx = it.x;
                             cphase = S.st->phase;
                             c.n = S.st->s_base + a.step + 1;
@@ -913,7 +986,7 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
                             c.scale = S.scale;
                             c.inv_scale = S.inv_scale;
                             c.phys = S.P;
-                            cred = cphase < PH_DONE && step_reduces(a, S.c, cphase, c.n) ? 1 : 0;
+                            cred = cphase < PH_DONE && (a.bit >= 0 ? (S.st->redm >> a.bit) & 1ull : step_reduces(a, S.c, cphase, c.n)) ? 1 : 0;
                             if (cphase < PH_DONE && ((reinterpret_cast<uintptr_t>(c.A) | (uintptr_t)c.P * sizeof(T)) & 15u)) {
                                 // not a legal bulk copy (lattices are allocated
                                 // aligned and planes padded to 64 slots, so this
@@ -995,7 +1068,7 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
                 int w = *static_cast<volatile int *>(&slot[s].item);
                 if (w < 0 && (int)blockIdx.x < nwork) w = blockIdx.x;
                 if (w >= 0) {
-                    const Solve3 &S = a.solves[a.work[w].x];
+                    const Solve3 &S = solves[item_of(w).x];
                     S.st->status = STATUS_WAIT_TIMEOUT;
                     S.st->phase = PH_ERR;
                     __threadfence();
@@ -1030,7 +1103,7 @@ __global__ void __launch_bounds__(ODD_BULK_THREADS, MINB) step3d_odd_bulk_kernel
                 ST::st2(A + (opp3(k) * P + i0), g[k].x, g[k].y, dir_bits(h0, k), dir_bits(h1, k));
         }
         if (red) {
-            const Solve3 &S = a.solves[solve];
+            const Solve3 &S = solves[solve];
             canonical_acc<TPB, BAR>(su, u, tid, tstart, nf, acc);
             finish_tile<TPB, BAR>(S, (int)(tstart / TV), n, acc, sh, defer_slot(a));
         }
@@ -1718,9 +1791,10 @@ __global__ void advance3d_kernel(Solve3 *solves, int nsolves, long long steps);
 // Deferred reduction of the launches with relative steps step0 .. step0 +
 // nsteps - 1 (nsteps <= DEFER_SLOTS, within one block of DEFER_SLOTS): the
 // fluxes (qbuf: per solve and step, q[3] and a flag), then the controllers
-// in step order.  mode: StepArgs::defer of those launches.
+// in step order.  mode: StepArgs::defer of those launches.  advance: then
+// move the running solves' s_base by it (the end of a chunk).
 cudaError_t launch_deferred3d(const Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
-                              int mode, cudaStream_t s);
+                              int mode, long long advance, cudaStream_t s);
 
 // Initial state: every population at rest (f = w, or h = 0 when shifted).
 template <class ST>

@@ -20,6 +20,7 @@
 #include "engine3d.cuh"
 #include "engine_md.cuh"
 #include "engine_host.h"
+#include "step3d_slots.cuh"
 
 using namespace lbm;
 
@@ -106,19 +107,28 @@ static int capture(lbm_batch *b)
     // Deferred reduction: a pass after every DEFER_SLOTS launches and at the
     // chunk's end; solves sit at different step counts, so their phases can
     // change inside a pass (mode 2)
+    const bool slots = lbm_slots_variant(b->precision, b->variant);
     for (int i = 0; i < b->chunk && e == cudaSuccess; ++i) {
-        a.step = i;
-        ae.step = i;
         const bool odd = ((i + 1) & 1) == 1;
-        e = lbm_launch_step(b->precision, b->variant, b->w1, odd, odd ? grid : grid_e, ctx->stream, odd ? a : ae);
+        StepArgs x = odd ? a : ae;
+        x.step = i;
+        if (slots) {
+            x.bit = i % DEFER_SLOTS;
+            x.n4 = (b->chunk & 3) == 0 ? (i + 1) & 3 : -1;   // every s_base is a multiple of the chunk
+            e = launch_slots3d_list(b->precision, is_pull_variant(b->precision, b->variant), b->w1, odd,
+                                    odd ? grid : grid_e, ctx->stream, x);
+        } else {
+            e = lbm_launch_step(b->precision, b->variant, b->w1, odd, odd ? grid : grid_e, ctx->stream, x);
+        }
         const bool pass_end = ((i + 1) % DEFER_SLOTS) == 0 || i + 1 == b->chunk;
         if (e == cudaSuccess && defer && pass_end) {
             const int first = i - (i % DEFER_SLOTS);
             e = launch_deferred3d(static_cast<const Solve3 *>(b->d_solves.p), std::max(1, b->slot_hi), first,
-                                  i + 1 - first, static_cast<double *>(b->d_qbuf.p), 2, ctx->stream);
+                                  i + 1 - first, static_cast<double *>(b->d_qbuf.p), 2,
+                                  i + 1 == b->chunk ? b->chunk : 0, ctx->stream);
         }
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && !defer) {
         advance3d_kernel<<<(b->cap_slots + 255) / 256, 256, 0, ctx->stream>>>(
             static_cast<Solve3 *>(b->d_solves.p), b->cap_slots, b->chunk);
         e = cudaGetLastError();
@@ -396,7 +406,7 @@ extern "C" int lbm_batch_submit3d(lbm_batch *b, const uint8_t *solid, int nx, in
         s.used = true;
         s.retired = false;
         s.bytes = lbm_lattice_bytes(s.S) + part_bytes;
-        lbm_init_state3(init[j], s.S.c);
+        lbm_init_state3(init[j], s.S.c, 2);
         CK(lbm_init_lattice(b->precision, s.S, ctx->stream));
         CK(cudaMemcpyAsync(s.S.st, &init[j], sizeof(State3), cudaMemcpyHostToDevice, ctx->stream));
     }

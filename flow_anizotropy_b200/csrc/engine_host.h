@@ -27,7 +27,8 @@ int lbm_default_batch_variant(int prec);
 // Deferred flux reduction (StepArgs::defer) for this precision, and the
 // doubles of a solve's partials buffer with it.
 bool lbm_defers(int prec);
-long long lbm_partial_doubles(int prec, int ntiles);
+// split: 8 partials per tile (Solve3::split).
+long long lbm_partial_doubles(int prec, int ntiles, bool split = false);
 bool lbm_is_device_ptr(const void *p);
 std::string &lbm_last_error_global();
 
@@ -71,12 +72,15 @@ long long lbm_lattice_bytes3d(long long nn, int prec);
 // Lattice bytes of one direction of a filled solve record (any storage form).
 long long lbm_lattice_bytes(const lbm::Solve3 &S);
 void lbm_fill_solve3(lbm::Solve3 &S, int nx, int ny, int nz, const double F[3], const lbm_params3d &p, int npt);
-void lbm_init_state3(lbm::State3 &st, const lbm::Ctl3 &c);
+// mode: StepArgs::defer of the launches (1 plain solves, 2 batches).
+void lbm_init_state3(lbm::State3 &st, const lbm::Ctl3 &c, int mode);
 int lbm_pick_npt(const lbm_params3d &p);
 // Pore-rank tables of a structure (wpre, fnode of S; nfluid, plane, ntiles for npt).
 int lbm_build_pores(lbm_ctx *ctx, lbm::Solve3 &S, int npt, DevMem &wpre, DevMem &fnode, DevMem &meta,
                     DevMem &meta2);
 int lbm_effective_variant(int prec, int variant, bool have_meta);
+// Does the (effective) variant run the kernels of step3d_slots.cuh?
+bool lbm_slots_variant(int prec, int variant);
 // Does the variant step a structure's directions in one work item (grouped work list)?
 bool lbm_grouped_variant(int prec, int variant);
 // ... and do all of its launches (the grouped pull form)?

@@ -1,7 +1,7 @@
 // FP64 D3Q19 kernels.  This translation unit is compiled with -fmad=false:
 // the collision keeps the reference's rounding step by step
 // (LMB3d/lbm3d-perm.cpp:218-245), so one step matches the CPU oracle bit for bit.
-#include "engine3d.cuh"
+#include "step3d_slots.cuh"
 
 namespace lbm {
 
@@ -39,6 +39,27 @@ cudaError_t launch_step3d_f64(int variant, bool w1, bool odd, dim3 grid, cudaStr
     if (w1) launch_f64<true>(vo, ve, odd, grid, s, a);
     else launch_f64<false>(vo, ve, odd, grid, s, a);
     return cudaGetLastError();
+}
+
+template <bool W1, bool EVEN>
+static cudaError_t launch_slots(bool split, int ntiles, int ndir, cudaStream_t s, const SlotArgs<false> &a)
+{
+    return split ? launch_pdl(step3d_aa_kernel<StoreF64, W1, EVEN, true, 128, 4, false>, dim3(4 * ntiles, ndir), 128, 0, s, a)
+                 : launch_pdl(step3d_aa_kernel<StoreF64, W1, EVEN, false, 256, 2, false>, dim3(ntiles, ndir), 256, 0, s, a);
+}
+
+cudaError_t launch_slots3d_f64(bool w1, bool odd, bool split, int ntiles, int ndir, cudaStream_t s, const SlotArgs<false> &a)
+{
+    return w1 ? (odd ? launch_slots<true, false>(split, ntiles, ndir, s, a) : launch_slots<true, true>(split, ntiles, ndir, s, a))
+              : (odd ? launch_slots<false, false>(split, ntiles, ndir, s, a) : launch_slots<false, true>(split, ntiles, ndir, s, a));
+}
+
+cudaError_t launch_slots3d_list_f64(bool w1, bool odd, dim3 grid, cudaStream_t s, const SlotArgs<true> &a)
+{
+    return w1 ? (odd ? launch_pdl(step3d_aa_kernel<StoreF64, true, false, false, 256, 2, true>, grid, 256, 0, s, a)
+                     : launch_pdl(step3d_aa_kernel<StoreF64, true, true, false, 256, 2, true>, grid, 256, 0, s, a))
+              : (odd ? launch_pdl(step3d_aa_kernel<StoreF64, false, false, false, 256, 2, true>, grid, 256, 0, s, a)
+                     : launch_pdl(step3d_aa_kernel<StoreF64, false, true, false, 256, 2, true>, grid, 256, 0, s, a));
 }
 
 int max_blocks_f64(int variant, bool odd)

@@ -2,7 +2,7 @@
 // (power-of-two scaled) or BF16, collision in FP32, flux reduced in FP64.
 #include <algorithm>
 
-#include "engine3d.cuh"
+#include "step3d_slots.cuh"
 
 namespace lbm {
 
@@ -17,7 +17,7 @@ int max_blocks_f64(int variant, bool odd);
 #define LBM_EVENG(ST, V, W) step3d_even_group_kernel<ST, even_lp(V).minb, W, even_meta(V)>
 #define LBM_EVENL(ST, V, W) step3d_even_links_kernel<ST, even_lp(V).minb, W, even_meta(V), even_pair(V)>
 #define LBM_EVENW(ST, V, W) step3d_even_links1_kernel<ST, even_lp(V).minb, W, even_meta(V)>
-#define LBM_ODDB(ST, W) step3d_odd_bulk_kernel<ST, odd_lp(4).minb, W>
+#define LBM_ODDB(ST, W, L) step3d_odd_bulk_kernel<ST, odd_lp(4).minb, W, L>
 #define LBM_PULL(ST, Q, W) step3d_pull_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
 #define LBM_PULL1(ST, Q, W) step3d_pull1_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
 #define LBM_PULLG(ST, Q, W) step3d_pull_group_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
@@ -44,11 +44,13 @@ template <class ST, bool W>
 static int prepare_bulk(int dev)
 {
     using T = typename ST::T;
-    const void *k = (const void *)LBM_ODDB(ST, W);
+    const void *k[2] = {(const void *)LBM_ODDB(ST, W, false), (const void *)LBM_ODDB(ST, W, true)};
     const unsigned smem = odd_bulk_smem<T>();
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     int nb = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, ODD_BULK_THREADS, smem) != cudaSuccess) return 0;
+    for (const void *f : k) {
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, ODD_BULK_THREADS, smem) != cudaSuccess) return 0;
+    }
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     g_bulk_ctas[ST::code - 1][W ? 1 : 0][dev] = nb * sms;
     return nb;
@@ -63,16 +65,15 @@ cudaError_t prepare_step3d_lp(int dev)
     return ok ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
-template <class ST, bool W>
-static cudaError_t launch_bulk(dim3 grid, cudaStream_t s, const StepArgs &a)
+template <class ST, bool W, bool L>
+static cudaError_t launch_bulk(dim3 grid, cudaStream_t s, const SlotArgs<L> &a)
 {
     int dev = 0;
     cudaGetDevice(&dev);
     const int ctas = (dev >= 0 && dev < 64) ? g_bulk_ctas[ST::code - 1][W ? 1 : 0][dev] : 0;
     if (ctas <= 0) return cudaErrorInvalidConfiguration;   // prepare_step3d_lp not run on this device
     grid.x = std::min<unsigned>(grid.x, (unsigned)ctas);
-    LBM_ODDB(ST, W)<<<grid, ODD_BULK_THREADS, odd_bulk_smem<typename ST::T>(), s>>>(a);
-    return cudaSuccess;
+    return launch_pdl(LBM_ODDB(ST, W, L), grid, ODD_BULK_THREADS, odd_bulk_smem<typename ST::T>(), s, a);
 }
 
 template <class ST, bool W>
@@ -98,7 +99,7 @@ static cudaError_t launch_lp(int v, bool odd, dim3 grid, cudaStream_t s, const S
         case 2: LBM_ODD(ST, 2, W)<<<grid, TPB, 0, s>>>(a); break;
         case 3: LBM_ODDP(ST, W)<<<grid, TPB, 0, s>>>(a); break;
         default: {
-            const cudaError_t e = launch_bulk<ST, W>(grid, s, a);
+            const cudaError_t e = launch_bulk<ST, W, true>(grid, s, SlotArgs<true>{a});
             if (e != cudaSuccess) return e;
         } break;
         }
@@ -122,6 +123,54 @@ static cudaError_t launch_lp(int v, bool odd, dim3 grid, cudaStream_t s, const S
         }
     }
     return cudaGetLastError();
+}
+
+// Step of a single solve whose records travel in the launch (variants with
+// slots_variant): the pull form, or the bulk-staged odd and grouped link-slot
+// even steps.  a.a.nwork: items of the bulk-staged launch.
+template <class ST, bool W>
+static cudaError_t launch_slots_lp(bool pull, bool odd, bool split, int ntiles, int ndir, cudaStream_t s, SlotArgs<false> a)
+{
+    if (pull)
+        return split ? launch_pdl(step3d_pull_slots_kernel<ST, W, true, 128, 6, false>, dim3(2 * ntiles, ndir), 128, 0, s, a)
+                     : launch_pdl(step3d_pull_slots_kernel<ST, W, false, 256, 3, false>, dim3(ntiles, ndir), 256, 0, s, a);
+    if (odd) {
+        a.a.nwork = ntiles * ndir;
+        return launch_bulk<ST, W, false>(dim3(a.a.nwork), s, a);
+    }
+    return split ? launch_pdl(step3d_links_slots_kernel<ST, W, true, 256, 4, false>, dim3(2 * ntiles), 256, 0, s, a)
+                 : launch_pdl(step3d_links_slots_kernel<ST, W, false, 256, 4, false>, dim3(ntiles), 256, 0, s, a);
+}
+
+cudaError_t launch_slots3d_lp(int prec, bool pull, bool w1, bool odd, bool split, int ntiles, int ndir, cudaStream_t s,
+                              const SlotArgs<false> &a)
+{
+    switch (prec) {
+    case 1: return w1 ? launch_slots_lp<StoreF32, true>(pull, odd, split, ntiles, ndir, s, a) : launch_slots_lp<StoreF32, false>(pull, odd, split, ntiles, ndir, s, a);
+    case 2: return w1 ? launch_slots_lp<StoreF16, true>(pull, odd, split, ntiles, ndir, s, a) : launch_slots_lp<StoreF16, false>(pull, odd, split, ntiles, ndir, s, a);
+    case 3: return w1 ? launch_slots_lp<StoreBF16, true>(pull, odd, split, ntiles, ndir, s, a) : launch_slots_lp<StoreBF16, false>(pull, odd, split, ntiles, ndir, s, a);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template <class ST, bool W>
+static cudaError_t launch_list_lp(bool pull, bool odd, dim3 grid, cudaStream_t s, const SlotArgs<true> &a)
+{
+    if (pull) return launch_pdl(step3d_pull_slots_kernel<ST, W, false, 256, 3, true>, grid, 256, 0, s, a);
+    if (odd) return launch_bulk<ST, W, true>(grid, s, a);
+    return launch_pdl(step3d_links_slots_kernel<ST, W, false, 256, 4, true>, grid, 256, 0, s, a);
+}
+
+cudaError_t launch_slots3d_list(int prec, bool pull, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &args)
+{
+    const SlotArgs<true> a{args};
+    switch (prec) {
+    case 0: return launch_slots3d_list_f64(w1, odd, grid, s, a);
+    case 1: return w1 ? launch_list_lp<StoreF32, true>(pull, odd, grid, s, a) : launch_list_lp<StoreF32, false>(pull, odd, grid, s, a);
+    case 2: return w1 ? launch_list_lp<StoreF16, true>(pull, odd, grid, s, a) : launch_list_lp<StoreF16, false>(pull, odd, grid, s, a);
+    case 3: return w1 ? launch_list_lp<StoreBF16, true>(pull, odd, grid, s, a) : launch_list_lp<StoreBF16, false>(pull, odd, grid, s, a);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_step3d_lp(int prec, int variant, bool w1, bool odd, dim3 grid, cudaStream_t s, const StepArgs &a)

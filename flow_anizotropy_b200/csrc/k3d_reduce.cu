@@ -11,31 +11,39 @@
 
 namespace lbm {
 
-// mode 1: the solves keep their phase through the pass (the single-solve
-// loop splits runs where the controller can act); mode 2: a phase can change
-// inside the pass, and every step the step kernels may have reduced is summed
-// (deferred_reduces).
-__global__ void __launch_bounds__(TPB) reduce3d_kernel(const Solve3 *solves, long long step0, double *qbuf, int mode)
+// The steps of a pass that were reduced are the bits of State3::redm, noted by
+// the controller pass before it (or with the initial state).
+__global__ void __launch_bounds__(TPB) reduce3d_kernel(const Solve3 *solves, long long step0, double *qbuf)
 {
     __shared__ double sh[TPB / 32][3];
     const int j = blockIdx.x, r = blockIdx.y;
     const Solve3 &S = solves[j];
     double *out = qbuf + 4ll * ((long long)j * DEFER_SLOTS + r);
-    const int phase = S.st->phase;
-    const long long rel = step0 + r;
-    const long long s_base = S.st->s_base;
-    const long long n = s_base + rel + 1;
-    const long long pass_start = s_base + (step0 & ~(long long)(DEFER_SLOTS - 1));
-    if (phase >= PH_DONE || !deferred_reduces(S.c, phase, n, pass_start, mode)) {
+    pdl_launch();
+    pdl_wait();
+    if (S.st->phase >= PH_DONE || !((S.st->redm >> r) & 1ull)) {
         if (threadIdx.x == 0) out[3] = 0.0;
         return;
     }
-    const double *p = S.partials + 3ll * (long long)(rel & (DEFER_SLOTS - 1)) * S.ntiles;
+    const int per = S.split ? TPB / 32 : 1;      // a split tile left its 8 warps' sums: add them as a block would
+    const double *p = S.partials + 3ll * (long long)((step0 + r) & (DEFER_SLOTS - 1)) * S.ntiles * per;
     double v[3] = {0.0, 0.0, 0.0};
     for (int t = threadIdx.x; t < S.ntiles; t += TPB) {
-        v[0] += p[3ll * t];
-        v[1] += p[3ll * t + 1];
-        v[2] += p[3ll * t + 2];
+        double x[3];
+        if (S.split) {
+            const double *w = p + 3ll * per * t;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                x[c] = 0.0;
+#pragma unroll
+                for (int q = 0; q < TPB / 32; ++q) x[c] += w[3 * q + c];
+            }
+        } else {
+            x[0] = p[3ll * t]; x[1] = p[3ll * t + 1]; x[2] = p[3ll * t + 2];
+        }
+        v[0] += x[0];
+        v[1] += x[1];
+        v[2] += x[2];
     }
     block_sum3<TPB>(v, sh);
     if (threadIdx.x == 0) {
@@ -50,44 +58,72 @@ __global__ void __launch_bounds__(TPB) reduce3d_kernel(const Solve3 *solves, lon
 // One block per solve: the pass's fluxes come to shared memory together,
 // then one thread runs the controller over the steps in order on a shared
 // copy of the state (the controller acts on a step when the phase it has
-// reached by then needs that step).
+// reached by then needs that step: which steps phase 1 needs is found by all
+// threads at once, the 64-bit divisions of one thread for 64 steps took most
+// of the pass).  The pass ends by noting, one thread per step, which of the
+// next DEFER_SLOTS steps reduce (State3::redm), so that the step kernels test
+// one bit, and with advance != 0 moves s_base on.
+static_assert(DEFER_SLOTS == 64, "two warps, one bit of a 64-bit mask per thread");
+__device__ __forceinline__ unsigned long long ballot64(unsigned (&bits)[2], bool x)
+{
+    const unsigned m = __ballot_sync(0xffffffffu, x);
+    if ((threadIdx.x & 31) == 0) bits[threadIdx.x >> 5] = m;
+    __syncthreads();
+    const unsigned long long r = (unsigned long long)bits[1] << 32 | bits[0];
+    __syncthreads();
+    return r;
+}
+
 __global__ void __launch_bounds__(DEFER_SLOTS) control3d_kernel(const Solve3 *solves, long long step0, int nsteps,
-                                                                  const double *qbuf)
+                                                                  const double *qbuf, int mode, long long advance)
 {
     __shared__ double q[DEFER_SLOTS][4];
     __shared__ State3 st;
+    __shared__ unsigned bits[2];
     const int j = blockIdx.x;
     const Solve3 &S = solves[j];
+    pdl_launch();
+    pdl_wait();
     for (int r = threadIdx.x; r < nsteps; r += blockDim.x)
         for (int c = 0; c < 4; ++c) q[r][c] = qbuf[4ll * ((long long)j * DEFER_SLOTS + r) + c];
     if (threadIdx.x == 0) st = *S.st;
     __syncthreads();
-    if (threadIdx.x != 0 || st.phase >= PH_DONE) return;
-    for (int r = 0; r < nsteps; ++r) {
-        if (st.phase >= PH_DONE) break;
-        const long long n = st.s_base + step0 + r + 1;
-        if (!needs_reduction(S.c, st.phase, n)) continue;
-        if (q[r][3] == 0.0) {            // a needed step without partials: cannot happen by construction
-            st.status = STATUS_WAIT_TIMEOUT;
-            st.phase = PH_ERR;
-            st.steps = n;
-            break;
+    if (st.phase >= PH_DONE) return;
+    const long long first = st.s_base + step0 + 1;
+    const unsigned long long run = ballot64(bits, (int)threadIdx.x < nsteps && needs_reduction(S.c, PH_RUN, first + threadIdx.x));
+    if (threadIdx.x == 0)
+        for (int r = 0; r < nsteps && st.phase < PH_DONE; ++r) {
+            if (st.phase == PH_RUN) {
+                const unsigned long long rest = run >> r;
+                if (!rest) break;
+                r += __ffsll((long long)rest) - 1;
+            }
+            const long long n = first + r;
+            if (q[r][3] == 0.0) {            // a needed step without partials: cannot happen by construction
+                st.status = STATUS_WAIT_TIMEOUT;
+                st.phase = PH_ERR;
+                st.steps = n;
+                break;
+            }
+            controller3(S.c, st, n, q[r]);
         }
-        controller3(S.c, st, n, q[r]);
-    }
+    __syncthreads();
+    const long long done = first + nsteps - 1;
+    const unsigned long long next = ballot64(bits, deferred_reduces(S.c, st.phase, done + threadIdx.x + 1, done, mode));
+    if (threadIdx.x != 0) return;
+    st.redm = next;
+    if (st.phase < PH_DONE) st.s_base += advance;
     *S.st = st;
 }
 
 cudaError_t launch_deferred3d(const Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
-                              int mode, cudaStream_t s)
+                              int mode, long long advance, cudaStream_t s)
 {
     if (nsolves <= 0 || nsteps <= 0) return cudaSuccess;
     if (nsteps > DEFER_SLOTS) return cudaErrorInvalidValue;
-    reduce3d_kernel<<<dim3(nsolves, nsteps), TPB, 0, s>>>(solves, step0, qbuf, mode);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_pdl(reduce3d_kernel, dim3(nsolves, nsteps), TPB, 0, s, solves, step0, qbuf);
     if (e != cudaSuccess) return e;
-    control3d_kernel<<<nsolves, DEFER_SLOTS, 0, s>>>(solves, step0, nsteps, qbuf);
-    return cudaGetLastError();
+    return launch_pdl(control3d_kernel, dim3(nsolves), DEFER_SLOTS, 0, s, solves, step0, nsteps, (const double *)qbuf, mode, advance);
 }
 
 }  // namespace lbm
