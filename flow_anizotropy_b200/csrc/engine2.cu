@@ -35,6 +35,9 @@ void fill_solve2(Solve2 &S, int nx, int ny, const double F[2], const lbm_params2
     // the reference stores fx, fy and tau in float globals (LMB2d/lbm.cpp:82-86,
     // LMB2d/main.cpp:104-106)
     S.fx = (float)F[0]; S.fy = (float)F[1]; S.tau = (float)p.tau;
+    // the loop-invariant pieces of the collision, rounded to float as there
+    volatile float fxt = S.fx * S.tau, fyt = S.fy * S.tau, itau = 1.0f / S.tau;
+    S.fxt = fxt; S.fyt = fyt; S.itau = itau;
     Ctl2 &c = S.c;
     c.eps = p.eps; c.qfloor = p.qfloor; c.ksigma = p.ksigma;
     c.lag = p.lag; c.min_steps = p.min_steps; c.max_steps = p.max_steps;
@@ -57,18 +60,19 @@ void init_state2(State2 &st, const Ctl2 &c)
 // The host loop of LMB2d/main.cpp:99-235 with the controller on the device:
 // launch up to the next step at which some direction's controller can change
 // phase, then read the states back.  The launches in between are replayed
-// from a CUDA graph of kGraphSteps step launches (plus the s_base advance),
+// from a CUDA graph of CHUNK2 step launches (plus the s_base advance),
 // which removes most of the per-launch overhead of this small, launch-bound
 // lattice; the step numbers and kernels are the same as single launches.
-constexpr int kGraphSteps = 100;
 
 static int run_plain2d(lbm_ctx *ctx, std::vector<Solve2> &hs, Solve2 *d_solves, State2 *d_states,
-                       const int2 *d_work, int nwork, std::vector<State2> &hst)
+                       std::vector<State2> &hst)
 {
     const int n = (int)hs.size();
     long long s = 0, base = 0;        // steps done; s_base of every solve (host copy)
     StepArgs2 a;
-    a.solves = d_solves; a.work = d_work; a.nwork = nwork;
+    a.solves = d_solves; a.step = 0; a.bit = -1;
+    const int ntiles = hs[0].ntiles;
+    bool masks = false;               // State2's step masks are those of s_base
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     struct GraphGuard {
@@ -91,33 +95,37 @@ static int run_plain2d(lbm_ctx *ctx, std::vector<Solve2> &hs, Solve2 *d_solves, 
             }
         }
         if (target == LLONG_MAX) break;
-        if (!exec && target - s >= kGraphSteps) {
+        if (!exec && target - s >= CHUNK2) {
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = cudaSuccess;
-            for (int i = 0; i < kGraphSteps && e == cudaSuccess; ++i) {
+            // launch i of a chunk runs step i + 1 after s_base (even)
+            for (int i = 0; i < CHUNK2 && e == cudaSuccess; ++i) {
                 StepArgs2 g = a;
                 g.step = i;
-                e = launch_step2d(dim3(nwork), ctx->stream, g);
+                g.bit = i;
+                e = launch_step2d((i & 1) == 0, ntiles, n, ctx->stream, g);
             }
-            if (e == cudaSuccess) e = launch_advance2d(d_solves, n, kGraphSteps, ctx->stream);
+            if (e == cudaSuccess) e = launch_advance2d(d_solves, n, CHUNK2, ctx->stream);
             const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
             CK(e);
             CK(e2);
             CK(cudaGraphInstantiate(&exec, graph, 0));
         }
         while (s < target) {
-            if (exec && target - s >= kGraphSteps) {
-                if (base != s) {
-                    // a chunk numbers its steps from s_base: catch up with the single steps
+            if (exec && (s & 1) == 0 && target - s >= CHUNK2) {
+                if (base != s || !masks) {
+                    // a chunk numbers its steps from s_base: catch up with the
+                    // single steps, and find the chunk's step flags
                     CK(launch_advance2d(d_solves, n, s - base, ctx->stream));
                     base = s;
+                    masks = true;
                 }
                 CK(cudaGraphLaunch(exec, ctx->stream));
-                s += kGraphSteps;
-                base += kGraphSteps;
+                s += CHUNK2;
+                base += CHUNK2;
             } else {
                 a.step = s - base;
-                CK(launch_step2d(dim3(nwork), ctx->stream, a));
+                CK(launch_step2d((s & 1) == 0, ntiles, n, ctx->stream, a));
                 ++s;
             }
         }
@@ -132,8 +140,7 @@ struct Set2 {
 };
 
 static int setup2d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, int ndir, const double *forces,
-                   const lbm_params2d &p, DevMem &mask, Set2 &set, DevMem &d_states, DevMem &d_solves,
-                   DevMem &d_work, int &nwork)
+                   const lbm_params2d &p, DevMem &mask, Set2 &set, DevMem &d_states, DevMem &d_solves)
 {
     long long npore = 0;
     int rc = lbm_upload_mask(ctx, solid, nx, ny, mask, npore);
@@ -143,7 +150,7 @@ static int setup2d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, int ndir,
     set.bufs.reserve(4 * ndir + 1);
     set.bufs.emplace_back(ctx->stream);                 // neighbour solid bits, shared by the directions
     DevMem &nbm = set.bufs.back();
-    CK(nbm.alloc(sizeof(uint16_t) * (size_t)nx * ny));
+    CK(nbm.alloc(sizeof(uint16_t) * ((size_t)nx * ny + 1)));      // read in pairs
     CK(launch_nbmask2d(static_cast<const uint32_t *>(mask.p), nx, ny, static_cast<uint16_t *>(nbm.p), ctx->stream));
     const uint16_t *nbm_p = static_cast<const uint16_t *>(nbm.p);
     CK(d_states.alloc(sizeof(State2) * ndir));
@@ -169,14 +176,8 @@ static int setup2d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, int ndir,
         init2d_kernel<<<256, 256, 0, ctx->stream>>>(S.A, S.plane, S.nn);
         CK(cudaGetLastError());
     }
-    std::vector<int2> work;
-    for (int j = 0; j < ndir; ++j)
-        for (int t = 0; t < set.hs[j].ntiles; ++t) work.push_back(make_int2(j, t));
-    nwork = (int)work.size();
     CK(d_solves.alloc(sizeof(Solve2) * ndir));
-    CK(d_work.alloc(sizeof(int2) * work.size()));
     CK(cudaMemcpyAsync(d_solves.p, set.hs.data(), sizeof(Solve2) * ndir, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(d_work.p, work.data(), sizeof(int2) * work.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(d_states.p, set.hst.data(), sizeof(State2) * ndir, cudaMemcpyHostToDevice, ctx->stream));
     return LBM_OK;
 }
@@ -193,13 +194,11 @@ extern "C" int lbm_solve2d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny,
     const lbm_params2d p = *params;
     int rc = check_params2d(ctx, p);
     if (rc) return rc;
-    DevMem mask(ctx->stream), d_states(ctx->stream), d_solves(ctx->stream), d_work(ctx->stream);
+    DevMem mask(ctx->stream), d_states(ctx->stream), d_solves(ctx->stream);
     Set2 set;
-    int nwork = 0;
-    rc = setup2d(ctx, solid, nx, ny, ndir, forces, p, mask, set, d_states, d_solves, d_work, nwork);
+    rc = setup2d(ctx, solid, nx, ny, ndir, forces, p, mask, set, d_states, d_solves);
     if (rc) return rc;
-    rc = run_plain2d(ctx, set.hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p),
-                     static_cast<const int2 *>(d_work.p), nwork, set.hst);
+    rc = run_plain2d(ctx, set.hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p), set.hst);
     if (rc) return rc;
 
     DevMem fr(ctx->stream);
@@ -266,7 +265,7 @@ extern "C" int lbm_solve2d_many(lbm_ctx *ctx, int nstruct, const uint8_t *solids
     std::vector<State2> hst(nsolve);
     std::vector<DevMem> bufs;
     bufs.reserve(4 * (size_t)nsolve);
-    DevMem d_states(ctx->stream), d_solves(ctx->stream), d_work(ctx->stream), fr(ctx->stream);
+    DevMem d_states(ctx->stream), d_solves(ctx->stream), fr(ctx->stream);
     CK(d_states.alloc(sizeof(State2) * nsolve));
     for (int k = 0; k < nstruct; ++k) {
         masks.emplace_back(ctx->stream);
@@ -277,7 +276,7 @@ extern "C" int lbm_solve2d_many(lbm_ctx *ctx, int nstruct, const uint8_t *solids
             return rc;
         }
         nbms.emplace_back(ctx->stream);
-        CK(nbms.back().alloc(sizeof(uint16_t) * (size_t)nn));
+        CK(nbms.back().alloc(sizeof(uint16_t) * ((size_t)nn + 1)));   // read in pairs
         CK(launch_nbmask2d(static_cast<const uint32_t *>(masks.back().p), nx, ny,
                            static_cast<uint16_t *>(nbms.back().p), ctx->stream));
         for (int j = 0; j < ndir; ++j) {
@@ -304,16 +303,10 @@ extern "C" int lbm_solve2d_many(lbm_ctx *ctx, int nstruct, const uint8_t *solids
             CK(cudaGetLastError());
         }
     }
-    std::vector<int2> work;
-    for (int id = 0; id < nsolve; ++id)
-        for (int t = 0; t < hs[id].ntiles; ++t) work.push_back(make_int2(id, t));
     CK(d_solves.alloc(sizeof(Solve2) * nsolve));
-    CK(d_work.alloc(sizeof(int2) * work.size()));
     CK(cudaMemcpyAsync(d_solves.p, hs.data(), sizeof(Solve2) * nsolve, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(d_work.p, work.data(), sizeof(int2) * work.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(d_states.p, hst.data(), sizeof(State2) * nsolve, cudaMemcpyHostToDevice, ctx->stream));
-    rc = run_plain2d(ctx, hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p),
-                     static_cast<const int2 *>(d_work.p), (int)work.size(), hst);
+    rc = run_plain2d(ctx, hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p), hst);
     if (rc) return rc;
     CK(fr.alloc(sizeof(double) * 2 * nsolve));
     CK(cudaMemsetAsync(fr.p, 0, sizeof(double) * 2 * nsolve, ctx->stream));
@@ -361,13 +354,11 @@ extern "C" int lbm_debug_steps2d(lbm_ctx *ctx, const uint8_t *solid, int nx, int
     p.avg_steps = 0; p.avg_sample = LLONG_MAX / 4; p.eps = 0.0; p.ksigma = 0.0;
     int rc = check_params2d(ctx, p);
     if (rc) return rc;
-    DevMem mask(ctx->stream), d_states(ctx->stream), d_solves(ctx->stream), d_work(ctx->stream);
+    DevMem mask(ctx->stream), d_states(ctx->stream), d_solves(ctx->stream);
     Set2 set;
-    int nwork = 0;
-    rc = setup2d(ctx, solid, nx, ny, 1, force, p, mask, set, d_states, d_solves, d_work, nwork);
+    rc = setup2d(ctx, solid, nx, ny, 1, force, p, mask, set, d_states, d_solves);
     if (rc) return rc;
-    rc = run_plain2d(ctx, set.hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p),
-                     static_cast<const int2 *>(d_work.p), nwork, set.hst);
+    rc = run_plain2d(ctx, set.hs, static_cast<Solve2 *>(d_solves.p), static_cast<State2 *>(d_states.p), set.hst);
     if (rc) return rc;
     const Solve2 &S = set.hs[0];
     if (f_out) {

@@ -65,7 +65,7 @@ constexpr size_t al256(size_t n) { return (n + 255) / 256 * 256; }
 // Byte layout of the scratch array.  Per direction: the AA lattice (9 planes),
 // the U,V snapshot and last fields, the per-tile flux partials.  Shared: the
 // bit mask (ceil(nx/32) * ny <= nx * ny words), the byte mask staged from
-// host memory, the neighbour solid bits (one 16-bit word per cell), controller states, solve records, the work list, and the
+// host memory, the neighbour solid bits (one 16-bit word per cell), controller states, solve records, and the
 // small sums (fieldres numerator/denominator per direction, pore count and
 // the non-binary flag of the mask packing).
 constexpr size_t kLatBytes = al256(sizeof(float) * Q2 * kCells);
@@ -75,10 +75,9 @@ constexpr size_t kDirBytes = kLatBytes + 2 * kFieldBytes + kPartBytes;
 constexpr size_t kMaskOff = kDirs * kDirBytes;
 constexpr size_t kSolidOff = kMaskOff + al256(sizeof(uint32_t) * kCells);
 constexpr size_t kNbmOff = kSolidOff + al256((size_t)kCells);
-constexpr size_t kStateOff = kNbmOff + al256(sizeof(uint16_t) * kCells);
+constexpr size_t kStateOff = kNbmOff + al256(sizeof(uint16_t) * (kCells + 1));   // read in pairs
 constexpr size_t kSolveOff = kStateOff + al256(sizeof(State2) * kDirs);
-constexpr size_t kWorkOff = kSolveOff + al256(sizeof(Solve2) * kDirs);
-constexpr size_t kSmallOff = kWorkOff + al256(sizeof(int2) * kDirs * kTiles);
+constexpr size_t kSmallOff = kSolveOff + al256(sizeof(Solve2) * kDirs);
 constexpr size_t kSmallBytes = al256(sizeof(double) * 2 * kDirs + 16);
 constexpr size_t kScratchBytes = kSmallOff + kSmallBytes;   // about 7 MB
 
@@ -156,11 +155,8 @@ extern "C" int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, i
     // per-direction solve records on the scratch
     auto *d_states = reinterpret_cast<State2 *>(base + kStateOff);
     auto *d_solves = reinterpret_cast<Solve2 *>(base + kSolveOff);
-    auto *d_work = reinterpret_cast<int2 *>(base + kWorkOff);
     Solve2 hs[kDirs];
     State2 hst[kDirs];
-    int2 work[kDirs * kTiles];
-    int nwork = 0;
     for (int j = 0; j < ndir; ++j) {
         Solve2 &S = hs[j];
         fill_solve2(S, nx, ny, forces + 2 * j, p);
@@ -180,16 +176,14 @@ extern "C" int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, i
         init_state2(hst[j], S.c);      // zero flux counter, phase RUN
         init2d_kernel<<<256, 256, 0, st>>>(S.A, S.plane, S.nn);
         CK(cudaGetLastError());
-        for (int t = 0; t < S.ntiles; ++t) work[nwork++] = make_int2(j, t);
     }
     CK(cudaMemcpyAsync(d_solves, hs, sizeof(Solve2) * ndir, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_work, work, sizeof(int2) * nwork, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_states, hst, sizeof(State2) * ndir, cudaMemcpyHostToDevice, st));
 
     // the host loop of lbm_solve2d: launch up to the next step at which some
     // direction's controller can change phase, then read the states back
     StepArgs2 a;
-    a.solves = d_solves; a.work = d_work; a.nwork = nwork;
+    a.solves = d_solves; a.bit = -1;
     for (long long s = 0;;) {
         CK(cudaMemcpyAsync(hst, d_states, sizeof(State2) * ndir, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -207,7 +201,7 @@ extern "C" int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, i
         if (target == LLONG_MAX) break;
         for (; s < target; ++s) {
             a.step = s;
-            CK(launch_step2d(dim3(nwork), st, a));
+            CK(launch_step2d((s & 1) == 0, hs[0].ntiles, ndir, st, a));
         }
     }
 

@@ -29,8 +29,16 @@ struct Ctl2 {              // LMB2d/main.cpp:64-79
     int hold;
 };
 
+// Steps per graph chunk of lbm_solve2d and lbm_solve2d_many, and of State2's
+// step masks.
+constexpr int CHUNK2 = 100, MASK2 = 128;
+static_assert(CHUNK2 <= MASK2 && CHUNK2 % 2 == 0, "a chunk's steps need a mask bit each and keep their parity");
+
 struct State2 {
     long long s_base;
+    // bit r: step s_base + 1 + r reduces the flux / keeps its velocities
+    // (advance2d_kernel; valid for a chunk, at whose end alone a phase changes)
+    unsigned long long redm[MASK2 / 64], keepm[MASK2 / 64];
     int phase, hold, have_prev, converged, status;
     unsigned counter;
     double pm[2], pse[2];
@@ -54,6 +62,7 @@ struct Solve2 {
     int ntiles;
     FastDiv dvx;
     float fx, fy, tau;     // as the reference's float globals (LMB2d/lbm.cpp:82-86)
+    float fxt, fyt, itau;  // fx * tau, fy * tau, 1 / tau, each rounded as the reference's expressions
     Ctl2 c;
     double *partials;      // ntiles * 2
     State2 *st;
@@ -63,9 +72,8 @@ struct Solve2 {
 
 struct StepArgs2 {
     const Solve2 *solves;
-    const int2 *work;
-    int nwork;
-    long long step;
+    long long step;        // steps completed = st->s_base + step
+    int bit;               // bit of State2's step masks, or -1: the step finds its flags itself
 };
 
 // Steps on which the flux is reduced, and on which the U,V field is kept.
@@ -180,14 +188,39 @@ __device__ __forceinline__ void block_sum2(double (&v)[2], double (*sh)[3])
     __syncthreads();
 }
 
-__device__ __forceinline__ void finish_tile2(const Solve2 &S, int tile, long long n,
-                                             double (&acc)[2], double (*sh)[3])
+// Threads of a step block: each steps the cell pair (2t, 2t + 1) of a tile of
+// TPB cells, and on reduction steps stands for threads t and t + THREADS2 of
+// a one-cell-per-thread block, whose order the flux sums keep.
+constexpr int THREADS2 = TPB / 2;
+
+// Sum over those TPB threads (block_sum2's order); result valid in thread 0.
+__device__ __forceinline__ void pair_sum2(double (&v)[2][2], double (*sh)[2])
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[h][k] += __shfl_down_sync(0xffffffffu, v[h][k], o);
+            if (lane == 0) sh[h * (THREADS2 / 32) + wid][k] = v[h][k];
+        }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a0 = 0.0, a1 = 0.0;
+        for (int w = 0; w < TPB / 32; ++w) { a0 += sh[w][0]; a1 += sh[w][1]; }
+        v[0][0] = a0; v[0][1] = a1;
+    }
+    __syncthreads();
+}
+
+__device__ __forceinline__ void finish_tile2(const Solve2 &S, int tile, long long n, double (&acc)[2][2], double (*sh)[2])
 {
     __shared__ int s_last;
-    block_sum2(acc, sh);
+    pair_sum2(acc, sh);
     if (threadIdx.x == 0) {
         double *p = S.partials + 2ll * tile;
-        p[0] = acc[0]; p[1] = acc[1];
+        p[0] = acc[0][0]; p[1] = acc[0][1];
         __threadfence();
         const unsigned prev = atomicAdd(&S.st->counter, 1u);
         s_last = (prev == (unsigned)S.ntiles - 1u);
@@ -195,58 +228,81 @@ __device__ __forceinline__ void finish_tile2(const Solve2 &S, int tile, long lon
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    double v[2] = {0.0, 0.0};
-    for (int t = threadIdx.x; t < S.ntiles; t += TPB) {
-        v[0] += __ldcg(S.partials + 2ll * t);
-        v[1] += __ldcg(S.partials + 2ll * t + 1);
-    }
-    block_sum2(v, sh);
+    double v[2][2] = {};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        for (int t = h * THREADS2 + threadIdx.x; t < S.ntiles; t += TPB) {
+            v[h][0] += __ldcg(S.partials + 2ll * t);
+            v[h][1] += __ldcg(S.partials + 2ll * t + 1);
+        }
+    pair_sum2(v, sh);
     if (threadIdx.x == 0) {
         State2 &st = *S.st;
         st.counter = 0u;
         // LMB2d/lbm.cpp:188-199: q_i = sum(u_i) / (L * L0^2), L0 = 4
-        const double q[2] = {v[0] / ((double)S.nx * 4.0 * 4.0), v[1] / ((double)S.ny * 4.0 * 4.0)};
+        const double q[2] = {v[0][0] / ((double)S.nx * 4.0 * 4.0), v[0][1] / ((double)S.ny * 4.0 * 4.0)};
         controller2(S.c, st, n, q);
     }
 }
 
-// macro + collision of one fluid node (LMB2d/lbm.cpp:563-612), in place on g;
-// returns the raw-moment velocity the reference stores in U, V.
-__device__ __forceinline__ void collide2(float (&g)[Q2], float fx, float fy, float tau,
-                                         float &U, float &V)
+// a / b per lane, correctly rounded, from y = RN(1/b) (see div_by).
+__device__ __forceinline__ float2 div_by2(float2 a, float2 b, float2 y)
 {
-    float rho = 0.0f;
+    const float2 nb = F32x2::neg(b);
+    float2 q = F32x2::mul(a, y);
+    q = F32x2::fma(F32x2::fma(nb, q, a), y, q);
+    return F32x2::fma(F32x2::fma(nb, q, a), y, q);
+}
+
+// macro + collision of two fluid nodes (LMB2d/lbm.cpp:563-612) in packed
+// FP32, in place on g; U, V the raw-moment velocities the reference stores.
+// Every value is rounded as the reference's operation order rounds it: terms
+// with a zero velocity component are skipped, opposite directions share what
+// is the same or exactly negated (e.u, 3 e.u, 4.5 (e.u)^2), and the four
+// quotients by rho share one reciprocal.  Sums with a product are written as
+// a difference from the negated product: the compiler contracts a packed
+// product into a packed sum (one rounding instead of two: 1 ulp in one
+// population of 589824 after 319 steps), whatever -fmad says, but not into
+// F32x2::sub, which is a multiply-add already.
+__device__ __forceinline__ void collide2(float2 (&g)[Q2], float fxt, float fyt, float itau, float2 &U, float2 &V)
+{
+    using O = F32x2;
+    float2 rho = g[0];
 #pragma unroll
-    for (int k = 0; k < Q2; ++k) rho = rho + g[k];
-    float ux = 0.0f, uy = 0.0f;
+    for (int k = 1; k < Q2; ++k) rho = O::add(rho, g[k]);
+    float2 ux = O::add(O::sub(O::sub(O::add(O::sub(g[1], g[3]), g[5]), g[6]), g[7]), g[8]);
+    float2 uy = O::sub(O::sub(O::add(O::add(O::sub(g[2], g[4]), g[5]), g[6]), g[7]), g[8]);
+    const float2 y = O::recip(rho);
+    U = ux = div_by2(ux, rho, y);
+    V = uy = div_by2(uy, rho, y);
+    ux = O::add(ux, div_by2(O::splat(fxt), rho, y));
+    uy = O::add(uy, div_by2(O::splat(fyt), rho, y));
+    const float2 usq = O::sub(O::mul(ux, ux), O::mul(O::neg(uy), uy));
+    const float2 base = O::sub(O::splat(1.0f), O::mul(O::splat(1.5f), usq));
+    auto relax = [&](float2 gk, float2 feq) { return O::sub(gk, O::mul(O::splat(itau), O::sub(gk, feq))); };
+    g[0] = relax(g[0], O::mul(O::mul(O::splat(w2(0)), rho), base));
+    const float2 wr[2] = {O::mul(O::splat(w2(1)), rho), O::mul(O::splat(w2(5)), rho)};
 #pragma unroll
-    for (int k = 0; k < Q2; ++k) {
-        if (ex2(k) == 1) ux = ux + g[k]; else if (ex2(k) == -1) ux = ux - g[k];
-        if (ey2(k) == 1) uy = uy + g[k]; else if (ey2(k) == -1) uy = uy - g[k];
-    }
-    ux = ux / rho;
-    uy = uy / rho;
-    U = ux; V = uy;
-    ux = ux + fx * tau / rho;
-    uy = uy + fy * tau / rho;
-    const float usq = ux * ux + uy * uy;
-    const float itau = 1.0f / tau;
-#pragma unroll
-    for (int k = 0; k < Q2; ++k) {
-        const float eu = (float)ex2(k) * ux + (float)ey2(k) * uy;
-        const float feq = (w2(k) * rho) * (((1.0f - 1.5f * usq) + 3.0f * eu) + (4.5f * eu) * eu);
-        g[k] = g[k] - itau * (g[k] - feq);
+    for (int p = 0; p < 4; ++p) {
+        constexpr int plus[4] = {1, 2, 5, 8};
+        const int k = plus[p], o = inv2(k);
+        const float2 eu = p == 0 ? ux : p == 1 ? uy : p == 2 ? O::add(ux, uy) : O::sub(ux, uy);
+        const float2 t3n = O::mul(O::splat(-3.0f), eu), t3 = O::mul(O::splat(3.0f), eu);
+        const float2 t45n = O::mul(O::mul(O::splat(-4.5f), eu), eu);
+        const float2 w = wr[p >> 1];
+        g[k] = relax(g[k], O::mul(w, O::sub(O::sub(base, t3n), t45n)));
+        g[o] = relax(g[o], O::mul(w, O::sub(O::sub(base, t3), t45n)));
     }
 }
 
-__global__ void __launch_bounds__(TPB, 4) step2d_kernel(const StepArgs2 a);
 __global__ void init2d_kernel(float *A, unsigned plane, int nn);
 // Neighbour solid bits of every cell (Solve2::nbm) from the bit mask.
 __global__ void nbmask2d_kernel(const uint32_t *mask, int nx, int ny, int wpr, uint16_t *nbm);
 __global__ void canon2d_kernel(const Solve2 S, long long done, float *f_out);
 __global__ void fieldres2d_kernel(const float *snap, const float *last, int nn, double *out);
 
-cudaError_t launch_step2d(dim3 grid, cudaStream_t s, const StepArgs2 &a);
+// One step of nsolves solves of one cell size, every one at step parity `odd`.
+cudaError_t launch_step2d(bool odd, int ntiles, int nsolves, cudaStream_t s, const StepArgs2 &a);
 cudaError_t launch_advance2d(const Solve2 *solves, int nsolves, long long steps, cudaStream_t s);
 cudaError_t launch_nbmask2d(const uint32_t *mask, int nx, int ny, uint16_t *nbm, cudaStream_t s);
 

@@ -5,68 +5,115 @@
 
 namespace lbm {
 
-__global__ void __launch_bounds__(TPB, 4) step2d_kernel(const StepArgs2 a)
+// AA slots of a cell's links (k = 1..8): population k is read from, and
+// population inv k written to, its own slot [k] across a solid link, else the
+// neighbour's slot [inv k] at x - e_k.
+__device__ __forceinline__ void slots2(const Solve2 &S, int nd, int x, int y, uint32_t sol, unsigned (&sl)[Q2])
 {
-    __shared__ double sh[TPB / 32][3];
-    for (int w = blockIdx.x; w < a.nwork; w += gridDim.x) {
-        const int2 item = a.work[w];
-        const Solve2 &S = a.solves[item.x];
-        State2 &st = *S.st;
-        if (st.phase >= PH_DONE) continue;
-        const long long n = st.s_base + a.step + 1;
-        const bool neighbour = (n & 1ll) == 0;
-        const bool red = reduce2(S.c, st, n);
-        const bool wsnap = snap2(S.c, st, n);
-        const bool wlast = last2(S.c, st, n);
-        float *__restrict__ A = S.A;
-        const unsigned P = S.plane;
-        double acc[2] = {0.0, 0.0};
-        const int nd = item.y * TPB + threadIdx.x;
-        if (nd < S.nn) {
-            const int y = S.dvx.div(nd);
-            const int x = nd - y * S.nx;
-            const int nx = S.nx, ny = S.ny;
-            const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
-            const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
-            const int X[3] = {xm, x, xp};
-            const int Yr[3] = {ym, y, yp};
-            const uint32_t sol = S.nbm[nd];
-            int idx[Q2];
+    const int nx = S.nx, ny = S.ny;
+    const int dx[3] = {x == 0 ? nx - 1 : -1, 0, x == nx - 1 ? 1 - nx : 1};
+    const int dy[3] = {y == 0 ? (ny - 1) * nx : -nx, 0, y == ny - 1 ? -(ny - 1) * nx : nx};
+    sl[0] = (unsigned)nd;
 #pragma unroll
-            for (int k = 0; k < Q2; ++k) idx[k] = Yr[ey2(k) + 1] * nx + X[ex2(k) + 1];
-            float U = 0.0f, V = 0.0f;
-            if (!(sol & 1u)) {
-                float g[Q2];
-                if (!neighbour) {
-#pragma unroll
-                    for (int k = 0; k < Q2; ++k) g[k] = A[k * P + (unsigned)nd];
-                } else {
-                    g[0] = A[(unsigned)nd];
-#pragma unroll
-                    for (int k = 1; k < Q2; ++k) {
-                        const int o = inv2(k);
-                        g[k] = ((sol >> o) & 1u) ? A[k * P + (unsigned)nd] : A[o * P + (unsigned)idx[o]];
-                    }
-                }
-                collide2(g, S.fx, S.fy, S.tau, U, V);
-                if (!neighbour) {
-#pragma unroll
-                    for (int k = 0; k < Q2; ++k) A[inv2(k) * P + (unsigned)nd] = g[k];
-                } else {
-                    A[(unsigned)nd] = g[0];
-#pragma unroll
-                    for (int k = 1; k < Q2; ++k) {
-                        if ((sol >> k) & 1u) A[inv2(k) * P + (unsigned)nd] = g[k];
-                        else A[k * P + (unsigned)idx[k]] = g[k];
-                    }
-                }
-                acc[0] = (double)U; acc[1] = (double)V;
-            }
-            if (wsnap) { S.snap[2 * nd] = U; S.snap[2 * nd + 1] = V; }
-            if (wlast) { S.last[2 * nd] = U; S.last[2 * nd + 1] = V; }
-        }
-        if (red) finish_tile2(S, item.y, n, acc, sh);
+    for (int k = 1; k < Q2; ++k) {
+        const int o = inv2(k);
+        sl[k] = ((sol >> o) & 1u) ? k * S.plane + (unsigned)nd : o * S.plane + (unsigned)(nd + dx[ex2(o) + 1] + dy[ey2(o) + 1]);
     }
+}
+
+// One step (odd: local, even: neighbour) of one tile of one solve.  A thread
+// steps an adjacent cell pair in packed FP32; all that does not change during
+// a solve (record, solid bits, slots) is read before the wait for the step
+// before, and the step's flags are bits of State2 (a 64-bit division per
+// thread and flag took a fifth of the step).  Bound by latency on one image
+// (512 blocks), by instructions on many.  Per step: one 256^2 image, both
+// directions, 5.3 -> 3.0 us; 16 images 58 (47 while averaging) -> 25 us.
+// (7 blocks of 72 registers per SM: with 8 of 64 the slots spill, 4.3 and 29.7 us.)
+template <bool ODD>
+__global__ void __launch_bounds__(THREADS2, 7) step2d_kernel(const StepArgs2 a)
+{
+    __shared__ double sh[TPB / 32][2];
+    __shared__ float su[2][TPB];
+    pdl_launch();
+    const Solve2 &S = a.solves[blockIdx.y];
+    const int tile = blockIdx.x, tid = threadIdx.x;
+    const int nd = tile * TPB + 2 * tid, nn = S.nn;
+    const unsigned P = S.plane;
+    float *__restrict__ A = S.A;
+    // solid bits of both cells (nd is even; the table is padded)
+    const uint32_t both = nd < nn ? *reinterpret_cast<const uint32_t *>(S.nbm + nd) : 0x00010001u;
+    const uint32_t s0 = both & 0xffffu, s1 = nd + 1 < nn ? both >> 16 : 1u;
+    const bool l0 = !(s0 & 1u), l1 = !(s1 & 1u);
+    unsigned sa[Q2], sb[Q2];
+    if constexpr (!ODD) {
+        const int y = S.dvx.div(nd), x = nd - y * S.nx;
+        const bool wrap = x + 1 == S.nx;
+        if (l0) slots2(S, nd, x, y, s0, sa);
+        if (l1) slots2(S, nd + 1, wrap ? 0 : x + 1, wrap ? y + 1 : y, s1, sb);
+    }
+    pdl_wait();
+    const State2 &st = *S.st;
+    const int phase = st.phase;
+    const long long n = st.s_base + a.step + 1;
+    bool red, keep;
+    if (a.bit >= 0) {
+        red = (st.redm[a.bit >> 6] >> (a.bit & 63)) & 1ull;
+        keep = (st.keepm[a.bit >> 6] >> (a.bit & 63)) & 1ull;
+    } else {
+        red = reduce2(S.c, st, n);
+        keep = snap2(S.c, st, n) || last2(S.c, st, n);
+    }
+    float2 g[Q2], U = make_float2(0.0f, 0.0f), V = U;
+    if constexpr (ODD) {
+        if (l0 || l1)
+#pragma unroll
+            for (int k = 0; k < Q2; ++k) g[k] = *reinterpret_cast<const float2 *>(A + (k * P + (unsigned)nd));
+    } else {
+#pragma unroll
+        for (int k = 0; k < Q2; ++k) {
+            g[k].x = l0 ? A[sa[k]] : w2(k);
+            g[k].y = l1 ? A[sb[k]] : w2(k);
+        }
+    }
+    if (phase >= PH_DONE) return;
+    if (l0 || l1) {
+        collide2(g, S.fxt, S.fyt, S.itau, U, V);
+        if constexpr (ODD) {
+            // a solid partner's slots are never read
+#pragma unroll
+            for (int k = 0; k < Q2; ++k) *reinterpret_cast<float2 *>(A + (inv2(k) * P + (unsigned)nd)) = g[k];
+        } else {
+#pragma unroll
+            for (int k = 0; k < Q2; ++k) {
+                if (l0) A[sa[inv2(k)]] = g[k].x;
+                if (l1) A[sb[inv2(k)]] = g[k].y;
+            }
+        }
+    }
+    if (!(red || keep)) return;
+    if (!l0) U.x = V.x = 0.0f;
+    if (!l1) U.y = V.y = 0.0f;
+    if (keep) {
+        const bool snap = snap2(S.c, st, n), last = last2(S.c, st, n);
+        if (nd < nn) {
+            if (snap) { S.snap[2 * nd] = U.x; S.snap[2 * nd + 1] = V.x; }
+            if (last) { S.last[2 * nd] = U.x; S.last[2 * nd + 1] = V.x; }
+        }
+        if (nd + 1 < nn) {
+            if (snap) { S.snap[2 * nd + 2] = U.y; S.snap[2 * nd + 3] = V.y; }
+            if (last) { S.last[2 * nd + 2] = U.y; S.last[2 * nd + 3] = V.y; }
+        }
+    }
+    if (!red) return;
+    su[0][2 * tid] = U.x; su[0][2 * tid + 1] = U.y;
+    su[1][2 * tid] = V.x; su[1][2 * tid + 1] = V.y;
+    __syncthreads();
+    double acc[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) acc[h][c] = (double)su[c][h * THREADS2 + tid];
+    finish_tile2(S, tile, n, acc, sh);
 }
 
 __global__ void nbmask2d_kernel(const uint32_t *mask, int nx, int ny, int wpr, uint16_t *nbm)
@@ -144,24 +191,46 @@ __global__ void fieldres2d_kernel(const float *snap, const float *last, int nn, 
     if (threadIdx.x == 0) { atomicAdd(out, v[0]); atomicAdd(out + 1, v[1]); }
 }
 
-// s_base += steps for every solve of a launch list (the step numbers of a
-// replayed chunk of step launches are relative to s_base)
-__global__ void advance2d_kernel(const Solve2 *solves, int nsolves, long long steps)
+// s_base += steps for every solve (the step numbers of a replayed chunk of
+// step launches are relative to s_base), and the flags of the next MASK2
+// steps, one thread per step.
+__global__ void __launch_bounds__(MASK2) advance2d_kernel(const Solve2 *solves, long long steps)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nsolves) solves[j].st->s_base += steps;
+    const Solve2 &S = solves[blockIdx.x];
+    pdl_launch();
+    pdl_wait();
+    State2 &st = *S.st;
+    const long long base = st.s_base + steps, n = base + 1 + threadIdx.x;
+    const bool run = st.phase < PH_DONE;
+    const unsigned red = __ballot_sync(0xffffffffu, run && reduce2(S.c, st, n));
+    const unsigned keep = __ballot_sync(0xffffffffu, run && (snap2(S.c, st, n) || last2(S.c, st, n)));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        reinterpret_cast<unsigned *>(st.redm)[threadIdx.x >> 5] = red;
+        reinterpret_cast<unsigned *>(st.keepm)[threadIdx.x >> 5] = keep;
+    }
+    if (threadIdx.x == 0) st.s_base = base;
 }
 
 cudaError_t launch_advance2d(const Solve2 *solves, int nsolves, long long steps, cudaStream_t s)
 {
-    advance2d_kernel<<<(nsolves + 127) / 128, 128, 0, s>>>(solves, nsolves, steps);
-    return cudaGetLastError();
+    return launch_pdl(advance2d_kernel, dim3(nsolves), MASK2, 0, s, solves, steps);
 }
 
-cudaError_t launch_step2d(dim3 grid, cudaStream_t s, const StepArgs2 &a)
+cudaError_t launch_step2d(bool odd, int ntiles, int nsolves, cudaStream_t s, const StepArgs2 &a)
 {
-    step2d_kernel<<<grid, TPB, 0, s>>>(a);
-    return cudaGetLastError();
+    if (nsolves > 65535) {
+        // beyond one grid's second dimension: a launch per 65535 solves
+        for (int j = 0; j < nsolves; j += 65535) {
+            StepArgs2 x = a;
+            x.solves += j;
+            const cudaError_t e = launch_step2d(odd, ntiles, nsolves - j < 65535 ? nsolves - j : 65535, s, x);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    const dim3 grid(ntiles, nsolves);
+    return odd ? launch_pdl(step2d_kernel<true>, grid, THREADS2, 0, s, a) : launch_pdl(step2d_kernel<false>, grid, THREADS2, 0, s, a);
 }
 
 }  // namespace lbm
