@@ -196,6 +196,9 @@ static lbm_params3d lbm_resolve_variant(lbm_params3d p)
     return p;
 }
 
+// Pore voxels x directions up to which a single 16-bit solve takes the pull form.
+constexpr long long SMALL_16BIT = 500000;
+
 static size_t elem_size(int prec) { return prec == LBM_FP64 ? 8 : (prec == LBM_FP32 ? 4 : 2); }
 
 long long lbm_plane_elems(long long nn) { return (nn + 63) / 64 * 64; }
@@ -486,17 +489,40 @@ static bool plain_split(int prec, int variant, const Solve3 &S, int ndir)
            (long long)S.ntiles * ndir <= (is_pull_variant(prec, variant) ? SPLIT_MAX_TILES_PULL : SPLIT_MAX_TILES);
 }
 
-// One step of the plain solves hs by the kernels of step3d_slots.cuh.
-static cudaError_t launch_plain_slots(const std::vector<Solve3> &hs, int prec, int variant, bool w1, const StepArgs &a, cudaStream_t s)
+// Directions of a single solve stepped together (slots variants): as many as
+// fit in L2 (126 MB) side by side, each group taking a chunk of steps in turn,
+// so that a step finds its lattices there instead of in DRAM.  Against all
+// three directions per step (us per step of all, B200): FP64 72^3 at 32 MB a
+// direction 36.9 -> 27.7 in pairs, 80^3 (56 MB) 65.3 -> 47.7 one at a time,
+// 96^3 (71 MB) 82.2 -> 69.2; FP32 (two lattices) 96^3 (71 MB) 42.1 -> 34.7,
+// 112^3 (102 MB) 62.6 -> 57.5.  A direction that does not fit gains nothing
+// (FP64 104^3, 98 MB: 113.7 -> 117.4; the pull form still does at 102 MB), and
+// where all fit together more of them fill the SMs better (FP64 64^3, 23 MB:
+// 20.8 together, 23.4 one at a time).  Two lattices a step apart hold 80 MB as
+// well as one does, but not 96 (FP64 72^3 with 100 MB allowed: 36.6).  The
+// 16-bit even step shares a voxel's link slots between the directions and is
+// not bound by DRAM (51 GLUPS in and out of L2), so it keeps them together.
+constexpr long long L2_GROUP_BYTES = 80ll << 20, L2_ONE_BYTES = 88ll << 20, L2_ONE_BYTES_PULL = 112ll << 20;
+static int plain_group(int prec, int variant, const Solve3 &S, int ndir)
+{
+    if (!lbm_slots_variant(prec, variant) || lbm_grouped_variant(prec, variant)) return ndir;
+    const long long one = lbm_lattice_bytes(S);
+    if (one > (S.pull ? L2_ONE_BYTES_PULL : L2_ONE_BYTES)) return ndir;
+    return (int)std::max(1ll, std::min<long long>(ndir, L2_GROUP_BYTES / one));
+}
+
+// One step of solves j0 .. j0 + nj - 1 of hs by the kernels of step3d_slots.cuh.
+static cudaError_t launch_plain_slots(const std::vector<Solve3> &hs, int j0, int nj, int prec, int variant, bool w1,
+                                      const StepArgs &a, cudaStream_t s)
 {
     const bool pull = is_pull_variant(prec, variant);
     // directions per launch: a structure's group where the even step is
     // grouped, else as many as the parameters hold
-    const int n = (int)hs.size(), per = lbm_grouped_variant(prec, variant) ? MAX_GROUP : MAX_PLAIN;
+    const int per = lbm_grouped_variant(prec, variant) ? MAX_GROUP : MAX_PLAIN;
     cudaError_t e = cudaSuccess;
-    for (int j = 0; j < n && e == cudaSuccess; j += per) {
+    for (int j = j0; j < j0 + nj && e == cudaSuccess; j += per) {
         SlotArgs<false> x;
-        const int m = std::min(per, n - j);
+        const int m = std::min(per, j0 + nj - j);
         for (int d = 0; d < m; ++d) x.s[d] = hs[j + d];
         x.a = a;
         const bool odd = a.n4 & 1;
@@ -546,16 +572,26 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
     ae.starve = a.starve;
     const bool gall = lbm_grouped_all(prec, variant);
     const bool slots = lbm_slots_variant(prec, variant);
-    auto launch = [&](long long rel, int n4, int bit) {
-        const bool odd = n4 & 1;
-        if (slots) {
-            StepArgs x = a;
-            x.step = rel; x.bit = bit; x.n4 = n4;
-            return launch_plain_slots(hs, prec, variant, w1, x, ctx->stream);
-        }
-        StepArgs x = (odd && !gall) ? a : ae;
-        x.step = rel;
-        return lbm_launch_step(prec, variant, w1, odd, dim3(x.nwork), ctx->stream, x);
+    const int group = plain_group(prec, variant, hs[0], n);
+    // `count` steps from relative step rel on (the step after s0 steps done, bit
+    // `bit` of the masks): every group of directions in turn takes all of
+    // them, so that its lattices stay in L2 from step to step
+    auto launch = [&](long long rel, long long s0, int bit, int count) {
+        cudaError_t e = cudaSuccess;
+        for (int j = 0; j < n && e == cudaSuccess; j += group)
+            for (int i = 0; i < count && e == cudaSuccess; ++i) {
+                const int n4 = (int)((s0 + i + 1) & 3);
+                const bool odd = n4 & 1;
+                StepArgs x = (slots || (odd && !gall)) ? a : ae;
+                x.step = rel + i;
+                if (slots) {
+                    x.bit = bit + i; x.n4 = n4;
+                    e = launch_plain_slots(hs, j, std::min(group, n - j), prec, variant, w1, x, ctx->stream);
+                } else {
+                    e = lbm_launch_step(prec, variant, w1, odd, dim3(x.nwork), ctx->stream, x);
+                }
+            }
+        return e;
     };
     // reduce and control the deferred single launches (before s_base moves,
     // before a chunk reuses their slots, and before the states are read)
@@ -583,9 +619,8 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
         if (target == LLONG_MAX) break;
         if (!exec && target - s >= 2 * kGraphSteps3) {
             CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = cudaSuccess;
             // launch i of a chunk runs step i + 1 after s_base (a multiple of 4)
-            for (int i = 0; i < kGraphSteps3 && e == cudaSuccess; ++i) e = launch(i, (i + 1) & 3, i);
+            cudaError_t e = launch(0, 0, 0, kGraphSteps3);
             if (e == cudaSuccess && defer) e = launch_deferred3d(d_solves, n, 0, kGraphSteps3, qb, 1, kGraphSteps3, ctx->stream);
             if (e == cudaSuccess && !defer) {
                 advance3d_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(d_solves, n, kGraphSteps3);
@@ -609,13 +644,17 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
                 s += kGraphSteps3;
                 base += kGraphSteps3;
             } else {
-                // every unfinished solve of the call is at step s + 1 (they start together)
-                CK(launch(s - base, (int)((s + 1) & 3), pending));
+                // every unfinished solve of the call is at step s + 1 (they start
+                // together); single launches up to the next chunk, pass or target
+                int count = 1;
                 if (defer) {
+                    while (count < DEFER_SLOTS - pending && s + count < target &&
+                           !(exec && ((s + count) & 3) == 0 && target - s - count >= kGraphSteps3)) ++count;
                     if (!pending) pend0 = s - base;
-                    if (++pending == DEFER_SLOTS) CK(flush());
                 }
-                ++s;
+                CK(launch(s - base, s, pending, count));
+                s += count;
+                if (defer && (pending += count) == DEFER_SLOTS) CK(flush());
             }
         }
         CK(flush());
@@ -637,13 +676,19 @@ extern "C" int lbm_solve3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, i
         return lbm_fail_input(ctx, "lattice too large (19 x nodes must stay below 2^32)");
     int rc = lbm_check_params3d(ctx, *params);
     if (rc) return rc;
-    const lbm_params3d p = lbm_resolve_variant(*params);
+    lbm_params3d p = lbm_resolve_variant(*params);
     const int prec = p.precision, npt = lbm_pick_npt(p);
 
     DevMem mask(ctx->stream);
     long long npore = 0;
     rc = lbm_upload_mask(ctx, solid, nx, (long long)ny * nz, mask, npore);
     if (rc) return rc;
+    // 16-bit storage: small structures are bound by the time of one short
+    // launch, where the pull form's single kernel is the faster one (three
+    // directions at porosity 0.5, us per step, pull / AA pair: 32^3 3.5 / 5.1,
+    // 48^3 4.3 / 6.4, 64^3 9.3 / 9.8, 80^3 17.1 / 16.3)
+    if (params->variant == LBM_VARIANT_DEFAULT && (prec == LBM_FP16 || prec == LBM_BF16) && npore * ndir <= SMALL_16BIT)
+        p.variant = NVAR_LP + 1;
 
     std::vector<Solve3> hs(ndir);
     std::vector<State3> hst(ndir);
@@ -912,7 +957,7 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
             x.step = s;
             if (slots) {
                 x.n4 = (int)((s + 1) & 3);
-                return launch_plain_slots(hs, precision, ev, true, x, ctx->stream);
+                return launch_plain_slots(hs, 0, ndir, precision, ev, true, x, ctx->stream);
             }
             return lbm_launch_step(precision, ev, true, odd, dim3(x.nwork), ctx->stream, x);
         };

@@ -43,7 +43,8 @@ extern "C" {
 
 /* lbm_params3d.variant: the library's default for the precision (the
  * variant the autotuner picks on the 128^3 tensor workload: FP32 76, FP16 and
- * BF16 150, 0 otherwise; a batch takes the same defaults).  Every variant of
+ * BF16 150, 0 otherwise; a batch takes the same defaults; lbm_solve3d runs
+ * small 16-bit structures, up to 500000 pore voxels x directions, as 76).  Every variant of
  * a precision gives the same
  * bits.  For FP32, FP16 and BF16, variants v < 75 are the in-place (AA)
  * lattice, odd-step kernel v / 15 and even-step kernel v % 15; v = 75..80

@@ -52,6 +52,20 @@ def test_split_limits(gpu, prec, n):
     _compare(_pores(n, (edge, edge, edge)), prec, 1, steps=(20, 12), velocity=False)
 
 
+@pytest.mark.parametrize("prec,n", [("fp64", 45 ** 3), ("fp64", 72 ** 3), ("fp64", 84 ** 3), ("fp32", 64 ** 3), ("fp32", 92 ** 3)])
+def test_direction_groups(gpu, prec, n):
+    """Lattices of a direction from a few MB to beyond L2: all directions in a
+    step, two of three (or of four), one at a time."""
+    edge = int(np.ceil((n / 0.8) ** (1 / 3)))
+    for ndir in (3, 4):
+        _compare(_pores(n, (edge, edge, edge)), prec, ndir, steps=(150, 33), velocity=False)
+
+
+@pytest.mark.parametrize("n", [166666, 166667])
+def test_small_16bit_limit(gpu, n):
+    _compare(_pores(n, (60, 60, 60)), "fp16", 3, steps=(70, 20))
+
+
 @pytest.mark.parametrize("steps", [(1, 0), (3, 2), (64, 0), (129, 1), (130, 64), (259, 130)])
 def test_step_counts(gpu, steps):
     _compare(_pores(900, (9, 11, 33), 3), "fp16", 3, steps=steps)
