@@ -295,12 +295,6 @@ cudaError_t lbm_launch_step(int prec, int variant, bool w1, bool odd, dim3 grid,
     return launch_step3d_lp(prec, variant, w1, odd, grid, s, a);
 }
 
-int lbm_max_blocks(int prec, int variant, bool odd)
-{
-    if (is_dense_m(prec)) return max_blocks_stepmd(variant);
-    return is_moment(prec) ? max_blocks_stepm(prec, variant) : max_blocks_step3d(prec, variant, odd);
-}
-
 cudaError_t lbm_init_lattice(int prec, const Solve3 &S, cudaStream_t s)
 {
     if (is_dense_m(prec)) return init_md_lattice(S, s);   // tensor maps; step 1 writes the records

@@ -1874,7 +1874,6 @@ cudaError_t launch_init3d(int prec, void *A, long long plane, long long n, cudaS
 // (once per device, before any launch or capture).
 cudaError_t prepare_step3d_lp(int dev);
 cudaError_t launch_canon3d(int prec, const Solve3 &S, long long done, double *f, float *u, cudaStream_t s);
-int max_blocks_step3d(int prec, int variant, bool odd);
 inline bool is_moment(int prec) { return prec == 4 || prec == 5; }
 inline bool is_dense_m(int prec) { return prec == 6; }
 // Dense moment form variants: z-segment length (planes per tile) x

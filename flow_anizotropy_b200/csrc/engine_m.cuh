@@ -239,6 +239,5 @@ __host__ __device__ constexpr int variant_m_minb(int v) { return v == 0 ? 3 : v 
 
 cudaError_t launch_stepm(int prec, int variant, dim3 grid, cudaStream_t s, const StepArgs &a);
 cudaError_t launch_canonm(int prec, const Solve3 &S, long long done, double *f, float *u, cudaStream_t s);
-int max_blocks_stepm(int prec, int variant);
 
 }  // namespace lbm

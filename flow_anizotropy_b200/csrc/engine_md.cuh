@@ -302,6 +302,5 @@ cudaError_t launch_canonmd(const Solve3 &S, long long done, double *f, float *u,
 cudaError_t launch_padmask(const Solve3 &S, cudaStream_t s);
 // Tensor maps (head of S.A) and zeroed records of one direction.
 cudaError_t init_md_lattice(const Solve3 &S, cudaStream_t s);
-int max_blocks_stepmd(int variant);
 
 }  // namespace lbm

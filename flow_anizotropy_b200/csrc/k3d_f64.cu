@@ -62,20 +62,6 @@ cudaError_t launch_slots3d_list_f64(bool w1, bool odd, dim3 grid, cudaStream_t s
                      : launch_pdl(step3d_aa_kernel<StoreF64, false, true, false, 256, 2, true>, grid, 256, 0, s, a));
 }
 
-int max_blocks_f64(int variant, bool odd)
-{
-    constexpr bool W1 = true;
-    variant = kernel_variant(0, variant);
-    const int vo = variant / NVAR_EVEN, ve = variant % NVAR_EVEN;
-    const void *k = odd ? (vo == 0 ? (const void *)LBM_ODD(0) : vo == 1 ? (const void *)LBM_ODD(1) : (const void *)LBM_ODD(2))
-                        : (ve == 0 ? (const void *)LBM_EVEN(0) : ve == 1 ? (const void *)LBM_EVEN(1)
-                           : ve == 2 ? (const void *)LBM_EVEN(2) : ve == 3 ? (const void *)LBM_EVEN(3)
-                           : ve == 4 ? (const void *)LBM_EVEN(0) : (const void *)LBM_EVEN(1));
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, TPB, 0);
-    return nb;
-}
-
 cudaError_t launch_init3d_f64(void *A, long long plane, long long n, cudaStream_t s)
 {
     init3d_kernel<StoreF64><<<1184, 256, 0, s>>>(A, plane, n);

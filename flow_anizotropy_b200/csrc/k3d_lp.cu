@@ -8,7 +8,6 @@ namespace lbm {
 
 cudaError_t launch_init3d_f64(void *A, long long plane, long long n, cudaStream_t s);
 cudaError_t launch_canon3d_f64(const Solve3 &S, long long done, double *f, float *u, cudaStream_t s);
-int max_blocks_f64(int variant, bool odd);
 
 #define LBM_ODD(ST, V, W) step3d_odd_kernel<ST, odd_lp(V).npt, odd_lp(V).minb, W>
 #define LBM_ODDP(ST, W) step3d_odd_pair_kernel<ST, odd_lp(3).minb, W>
@@ -21,20 +20,6 @@ int max_blocks_f64(int variant, bool odd);
 #define LBM_PULL(ST, Q, W) step3d_pull_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
 #define LBM_PULL1(ST, Q, W) step3d_pull1_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
 #define LBM_PULLG(ST, Q, W) step3d_pull_group_kernel<ST, pull_minb(Q), W, pull_meta(Q)>
-
-// Pull-form kernel of pull variant q (any step parity).
-template <class ST, bool W>
-static const void *pull_kernel(int q)
-{
-    switch (q) {
-    case 0: return (const void *)LBM_PULL(ST, 0, W);
-    case 1: return (const void *)LBM_PULL(ST, 1, W);
-    case 2: return (const void *)LBM_PULL(ST, 2, W);
-    case 3: return (const void *)LBM_PULL1(ST, 3, W);
-    case 4: return (const void *)LBM_PULLG(ST, 4, W);
-    default: return (const void *)LBM_PULLG(ST, 5, W);
-    }
-}
 
 // Persistent CTAs of the bulk-staged odd kernel per (storage, tau = 1, device),
 // set by prepare_bulk once its shared-memory ring has been allowed.
@@ -83,11 +68,12 @@ static cudaError_t launch_lp(int v, bool odd, dim3 grid, cudaStream_t s, const S
     if (v >= NVAR_LP) {
         switch (v - NVAR_LP) {
         case 0: LBM_PULL(ST, 0, W)<<<grid, TPB, 0, s>>>(a); break;
-        case 1: LBM_PULL(ST, 1, W)<<<grid, TPB, 0, s>>>(a); break;
+        // 1 runs step3d_pull_slots_kernel, or without neighbour records as 2
         case 2: LBM_PULL(ST, 2, W)<<<grid, TPB, 0, s>>>(a); break;
         case 3: LBM_PULL1(ST, 3, W)<<<grid, TPB, 0, s>>>(a); break;
         case 4: LBM_PULLG(ST, 4, W)<<<grid, TPB, 0, s>>>(a); break;
-        default: LBM_PULLG(ST, 5, W)<<<grid, TPB, 0, s>>>(a); break;
+        case 5: LBM_PULLG(ST, 5, W)<<<grid, TPB, 0, s>>>(a); break;
+        default: return cudaErrorInvalidValue;
         }
         return cudaGetLastError();
     }
@@ -181,47 +167,6 @@ cudaError_t launch_step3d_lp(int prec, int variant, bool w1, bool odd, dim3 grid
     case 2: return w1 ? launch_lp<StoreF16, true>(variant, odd, grid, s, a) : launch_lp<StoreF16, false>(variant, odd, grid, s, a);
     case 3: return w1 ? launch_lp<StoreBF16, true>(variant, odd, grid, s, a) : launch_lp<StoreBF16, false>(variant, odd, grid, s, a);
     default: return cudaErrorInvalidValue;
-    }
-}
-
-template <class ST>
-static int occ(int v, bool odd)
-{
-    if (v >= NVAR_LP) {
-        int nb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pull_kernel<ST, true>(v - NVAR_LP), TPB, 0);
-        return nb;
-    }
-    const int vo = v / NVAR_EVEN_LP, ve = v % NVAR_EVEN_LP;
-    if (odd && vo == 4) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        return prepare_bulk<ST, true>(dev);
-    }
-    const void *k = odd ? (vo == 0 ? (const void *)LBM_ODD(ST, 0, true) : vo == 1 ? (const void *)LBM_ODD(ST, 1, true)
-                           : vo == 2 ? (const void *)LBM_ODD(ST, 2, true) : (const void *)LBM_ODDP(ST, true))
-                        : (ve == 0 ? (const void *)LBM_EVEN(ST, 0, true) : ve == 1 ? (const void *)LBM_EVEN(ST, 1, true)
-                           : ve == 2 ? (const void *)LBM_EVEN(ST, 2, true) : ve == 3 ? (const void *)LBM_EVEN(ST, 3, true)
-                           : ve == 4 ? (const void *)LBM_EVENA(ST, 4, true) : ve == 5 ? (const void *)LBM_EVENA(ST, 5, true)
-                           : ve == 6 ? (const void *)LBM_EVENG(ST, 6, true) : ve == 7 ? (const void *)LBM_EVENG(ST, 7, true)
-                           : ve == 8 ? (const void *)LBM_EVENL(ST, 8, true) : ve == 9 ? (const void *)LBM_EVENL(ST, 9, true)
-                           : ve == 10 ? (const void *)LBM_EVENL(ST, 10, true) : ve == 11 ? (const void *)LBM_EVENL(ST, 11, true)
-                           : ve == 12 ? (const void *)LBM_EVENL(ST, 12, true) : ve == 13 ? (const void *)LBM_EVENW(ST, 13, true)
-                           : (const void *)LBM_EVENW(ST, 14, true));
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (!odd && even_wide(ve)) ? 2 * TPB : TPB, 0);
-    return nb;
-}
-
-int max_blocks_step3d(int prec, int variant, bool odd)
-{
-    variant = kernel_variant(prec, variant);
-    switch (prec) {
-    case 0: return max_blocks_f64(variant, odd);
-    case 1: return occ<StoreF32>(variant, odd);
-    case 2: return occ<StoreF16>(variant, odd);
-    case 3: return occ<StoreBF16>(variant, odd);
-    default: return 0;
     }
 }
 

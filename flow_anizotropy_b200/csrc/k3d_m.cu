@@ -24,21 +24,6 @@ cudaError_t launch_stepm(int prec, int variant, dim3 grid, cudaStream_t s, const
     return cudaErrorInvalidValue;
 }
 
-template <class MT>
-static int occ_m(int v)
-{
-    const void *k = v == 0 ? (const void *)LBM_M(MT, 0) : v == 1 ? (const void *)LBM_M(MT, 1)
-                                                                 : (const void *)LBM_M(MT, 2);
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, TPB, 0);
-    return nb;
-}
-
-int max_blocks_stepm(int prec, int variant)
-{
-    return prec == MomF32::code ? occ_m<MomF32>(variant) : occ_m<MomF64>(variant);
-}
-
 cudaError_t launch_canonm(int prec, const Solve3 &S, long long done, double *f, float *u, cudaStream_t s)
 {
     if (prec == MomF32::code) canonm_kernel<MomF32><<<1184, 256, 0, s>>>(S, done, f, u);

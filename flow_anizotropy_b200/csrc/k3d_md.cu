@@ -68,17 +68,6 @@ __global__ void padmask_kernel(const uint32_t *mask, int nx, int ny, int nz, int
 
 #define LBM_MD(V) stepmd_kernel<md_ns(V), md_minb(V)>
 
-static const void *md_kernel(int v)
-{
-    switch (v) {
-    case 0: return (const void *)LBM_MD(0);
-    case 1: return (const void *)LBM_MD(1);
-    case 2: return (const void *)LBM_MD(2);
-    case 3: return (const void *)LBM_MD(3);
-    default: return nullptr;
-    }
-}
-
 cudaError_t launch_stepmd(int v, dim3 grid, cudaStream_t s, const StepArgs &a)
 {
     const size_t smem = md_smem_bytes(v);
@@ -90,14 +79,6 @@ cudaError_t launch_stepmd(int v, dim3 grid, cudaStream_t s, const StepArgs &a)
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
-}
-
-int max_blocks_stepmd(int v)
-{
-    const void *k = md_kernel(v);
-    int nb = 0;
-    if (k) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, MD_TPB, md_smem_bytes(v));
-    return nb;
 }
 
 cudaError_t launch_canonmd(const Solve3 &S, long long done, double *f, float *u, cudaStream_t s)
