@@ -192,8 +192,8 @@ int lbm_solve2d_many(lbm_ctx *ctx, int nstruct, const uint8_t *solids, int nx, i
  * synchronises its stream and is not capturable.
  *   One array per device and process: overlapping calls on one device would
  * race on it, so they are serialised by a per-device lock.
- *   The time loop launches one step at a time from the host (about 8.6 us per
- * step on 256 x 256 against 6.8 us for lbm_solve2d's graph chunks). */
+ *   The time loop launches one step at a time from the host (about 3.9 us per
+ * step on 256 x 256 against 3.0 us for lbm_solve2d's graph chunks). */
 int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny,
                         int ndir, const double *forces, const lbm_params2d *params,
                         lbm_result2d *results, float *vel_out);
