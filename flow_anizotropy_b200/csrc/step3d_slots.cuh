@@ -21,7 +21,8 @@
 // 3.8 us, 64^3 28.2 -> 20.6, 80^3 74.0 -> 62.7 (86 % of the copy bandwidth);
 // FP32 pull 96^3 47.0 -> 41.2 (82 %), 97 x 61 x 75 with four directions 30.6
 // -> 23.7; BF16 128^3 62.8 -> 56.4; FP16 batch of eight structures 119.8 ->
-// 106.8.  What is left: FP64 and FP32 run near the copy bandwidth where the
+// 106.8 (all directions in every step; stepped in groups that fit L2, see
+// plain_group, 80^3 takes 47.7, 96^3 34.7 and 97 x 61 x 75 21).  What is left: FP64 and FP32 run near the copy bandwidth where the
 // lattices exceed L2; the 16-bit even step waits on its scattered accesses.
 #pragma once
 #include "engine3d.cuh"
