@@ -22,8 +22,9 @@
 // FP32 pull 96^3 47.0 -> 41.2 (82 %), 97 x 61 x 75 with four directions 30.6
 // -> 23.7; BF16 128^3 62.8 -> 56.4; FP16 batch of eight structures 119.8 ->
 // 106.8 (all directions in every step; stepped in groups that fit L2, see
-// plain_group, 80^3 takes 47.7, 96^3 34.7 and 97 x 61 x 75 21).  What is left: FP64 and FP32 run near the copy bandwidth where the
-// lattices exceed L2; the 16-bit even step waits on its scattered accesses.
+// plain_group, 80^3 takes 47.7, 96^3 34.7 and 97 x 61 x 75 22).  What is left:
+// FP64 and FP32 run near the copy bandwidth where the lattices exceed L2; the
+// 16-bit even step waits on its scattered accesses.
 #pragma once
 #include "engine3d.cuh"
 
