@@ -286,6 +286,10 @@ __device__ __forceinline__ void collide_pairs(typename O::V (&h)[Q3], const Phys
 // W: the word cp.async stages for one population (cp.async copies 4, 8 or 16
 // bytes, so a 2-byte population travels in the aligned 4-byte word that
 // holds it, and `unword` picks its half).
+// ld and ld2 go through overloads of __ldcs that are volatile asm (the plain
+// arithmetic types), never through the ones of __half and __nv_bfloat16, which
+// are plain asm: to the compiler a function of the address alone, that it may
+// move above a griddepcontrol.wait and so above the stores of the step before.
 struct StoreF64 {
     using T = double; using C = double; using W = double;
     __device__ static __forceinline__ const W *word(const T *p) { return p; }
@@ -336,7 +340,10 @@ struct StoreF16 {
     }
     static constexpr bool shifted = true;
     static constexpr int code = 2;
-    __device__ static __forceinline__ C ld(const T *p) { return __half2float(__ldcs(p)); }
+    __device__ static __forceinline__ C ld(const T *p)
+    {
+        return __half2float(__ushort_as_half(__ldcs(reinterpret_cast<const unsigned short *>(p))));
+    }
     __device__ static __forceinline__ void st(T *p, C v) { __stcs(p, __float2half_rn(v)); }
     // stochastic rounding (sm_100a cvt.rs with random bits; the product bits
     // in `rnd` are rotated so that its well-mixed high half is used): rounds up
@@ -391,7 +398,10 @@ struct StoreBF16 {
     }
     static constexpr bool shifted = true;
     static constexpr int code = 3;
-    __device__ static __forceinline__ C ld(const T *p) { return __bfloat162float(__ldcs(p)); }
+    __device__ static __forceinline__ C ld(const T *p)
+    {
+        return __bfloat162float(__ushort_as_bfloat16(__ldcs(reinterpret_cast<const unsigned short *>(p))));
+    }
     __device__ static __forceinline__ void st(T *p, C v) { __stcs(p, __float2bfloat16_rn(v)); }
     // stochastic rounding (as StoreF16)
     static constexpr bool stochastic = true;

@@ -162,7 +162,9 @@ template <> struct SlotArgs<false> { StepArgs a; Solve3 s[MAX_PLAIN]; };
 // Programmatic dependent launch: let the next grid's blocks start; wait until
 // every grid before this one has ended and its writes are visible.  Every
 // block waits before it reads what a step writes or returns, so the end of a
-// grid implies the end of all before it.
+// grid implies the end of all before it.  Both are volatile with a memory
+// clobber, so what must stay behind the wait has to be an ordinary access
+// (through a pointer that is not __restrict__) or volatile asm.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
