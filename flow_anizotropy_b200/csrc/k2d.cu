@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(THREADS2, 7) step2d_kernel(const StepArgs2 a)
     const int tile = blockIdx.x, tid = threadIdx.x;
     const int nd = tile * TPB + 2 * tid, nn = S.nn;
     const unsigned P = S.plane;
-    float *__restrict__ A = S.A;
+    float *A = S.A;
     // solid bits of both cells (nd is even; the table is padded)
     const uint32_t both = nd < nn ? *reinterpret_cast<const uint32_t *>(S.nbm + nd) : 0x00010001u;
     const uint32_t s0 = both & 0xffffu, s1 = nd + 1 < nn ? both >> 16 : 1u;

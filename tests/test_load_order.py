@@ -43,3 +43,12 @@ def test_population_loads_are_volatile(store):
     assert loads
     for fn, typ in loads:
         assert (typ or POINTER[store]) in volatile, f"{store}::{fn}"
+
+
+@pytest.mark.parametrize("source", ["k2d.cu", "step3d_slots.cuh", "k3d_reduce.cu"])
+def test_no_restrict_across_the_wait(source):
+    """An ordinary load stays behind the wait because the wait may write any
+    memory; a __restrict__ pointer declared before it would promise that what
+    it points to is written through it alone."""
+    code = re.sub(r"//.*", "", (CSRC / source).read_text())
+    assert "pdl_wait()" in code and "__restrict__" not in code
