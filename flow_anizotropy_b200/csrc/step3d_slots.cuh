@@ -335,11 +335,11 @@ __global__ void __launch_bounds__(NT, MINB) step3d_links_slots_kernel(const __gr
         for (int k = 0; k < Q3 - 1; ++k) sl[k][j * NT + tid] = q[k];
     }
     pdl_wait();
-    const int n4 = step_n4(S0, a);
     unsigned redm = 0;                 // split: directions that reduce
 #pragma unroll 1
     for (int d = 0; d < ng; ++d) {
         const Solve3 &S = Sp[d];
+        const int n4 = step_n4(S, a);  // the direction's own: a finished leader's step count stands still
         const T *R = slots_src<T>(S, n4);
         T *W = slots_dst<T>(S, n4);
         const StepHead h = step_head(S, a);
