@@ -136,6 +136,7 @@ struct Solve3 {
     int group;            // grouped even step: directions in the group led by this record (else 0)
     int pull;             // two-lattice pull form (step3d_pull_kernel): A and B alternate
     int split;            // flux partials per warp of a tile (step3d_slots.cuh), else per tile
+    int done;             // noted by control3d_kernel: the solve has finished (a batch's step kernels, step3d_slots.cuh)
     int aa2;              // two-lattice AA form: the even step scatters into the other lattice (aa_buf)
 };
 
@@ -1795,7 +1796,7 @@ __global__ void advance3d_kernel(Solve3 *solves, int nsolves, long long steps);
 // fluxes (qbuf: per solve and step, q[3] and a flag), then the controllers
 // in step order.  mode: StepArgs::defer of those launches.  advance: then
 // move the running solves' s_base by it (the end of a chunk).
-cudaError_t launch_deferred3d(const Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
+cudaError_t launch_deferred3d(Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
                               int mode, long long advance, cudaStream_t s);
 
 // Initial state: every population at rest (f = w, or h = 0 when shifted).

@@ -74,21 +74,27 @@ __device__ __forceinline__ unsigned long long ballot64(unsigned (&bits)[2], bool
     return r;
 }
 
-__global__ void __launch_bounds__(DEFER_SLOTS) control3d_kernel(const Solve3 *solves, long long step0, int nsteps,
+__global__ void __launch_bounds__(DEFER_SLOTS) control3d_kernel(Solve3 *solves, long long step0, int nsteps,
                                                                   const double *qbuf, int mode, long long advance)
 {
     __shared__ double q[DEFER_SLOTS][4];
     __shared__ State3 st;
     __shared__ unsigned bits[2];
     const int j = blockIdx.x;
-    const Solve3 &S = solves[j];
+    Solve3 &S = solves[j];
     pdl_launch();
     pdl_wait();
     for (int r = threadIdx.x; r < nsteps; r += blockDim.x)
         for (int c = 0; c < 4; ++c) q[r][c] = qbuf[4ll * ((long long)j * DEFER_SLOTS + r) + c];
     if (threadIdx.x == 0) st = *S.st;
     __syncthreads();
-    if (st.phase >= PH_DONE) return;
+    // for the step kernels' blocks, which may be reading it (noted_done); here
+    // too, since a batch's records are written anew when its work list changes
+    auto note_done = [&] { *static_cast<volatile int *>(&S.done) = 1; };
+    if (st.phase >= PH_DONE) {
+        if (threadIdx.x == 0) note_done();
+        return;
+    }
     const long long first = st.s_base + step0 + 1;
     const unsigned long long run = ballot64(bits, (int)threadIdx.x < nsteps && needs_reduction(S.c, PH_RUN, first + threadIdx.x));
     if (threadIdx.x == 0)
@@ -113,10 +119,11 @@ __global__ void __launch_bounds__(DEFER_SLOTS) control3d_kernel(const Solve3 *so
     if (threadIdx.x != 0) return;
     st.redm = next;
     if (st.phase < PH_DONE) st.s_base += advance;
+    else note_done();
     *S.st = st;
 }
 
-cudaError_t launch_deferred3d(const Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
+cudaError_t launch_deferred3d(Solve3 *solves, int nsolves, long long step0, int nsteps, double *qbuf,
                               int mode, long long advance, cudaStream_t s)
 {
     if (nsolves <= 0 || nsteps <= 0) return cudaSuccess;

@@ -12,7 +12,9 @@
 //   - all that does not change during a solve (item, record, neighbour
 //     records, row starts, slots) is read before griddepcontrol.wait, so that
 //     with programmatic launches it overlaps the end of the step before;
-//   - populations are requested before the solve's state has arrived;
+//   - populations are requested before the solve's state has arrived (a
+//     single solve launches its unfinished directions only; a batch lists
+//     finished solves until they are polled, their record says so);
 //   - whether a step reduces is one bit of State3::redm instead of a division
 //     of the 64-bit step number per thread, and the flux sums of steps that
 //     do not reduce are not formed.
@@ -148,6 +150,11 @@ __device__ __forceinline__ bool slots_item(const SlotArgs<LIST> &ka, const Solve
     return true;
 }
 
+// Does the record say that the solve has finished (control3d_kernel)?  Read
+// before the wait, so the note of a pass that is still running may be missed:
+// the solve's state, read after the wait, decides then.
+__device__ __forceinline__ bool noted_done(const Solve3 &S) { return *static_cast<const volatile int *>(&S.done) != 0; }
+
 // AA step, odd (local: slot k is the voxel's own, written with opp k) or even
 // (neighbour: link slots), one voxel per thread at a time: the voxel of a
 // split tile's thread, or voxels t and t + TPB of a whole tile.
@@ -164,6 +171,7 @@ __global__ void __launch_bounds__(NT, MINB) step3d_aa_kernel(const __grid_consta
     pdl_launch();
     if (!slots_item<LIST>(ka, Sp, tile, blockIdx.x / PARTS)) { pdl_wait(); return; }
     const Solve3 &S = *Sp;
+    if (LIST && noted_done(S)) { pdl_wait(); return; }
     const int part = blockIdx.x % PARTS;
     const unsigned P = (unsigned)S.plane, nf = (unsigned)S.nfluid;
     const unsigned i0 = (unsigned)tile * (TPB * TILE_NPT) + (SPLIT ? split_voxel<NT, 1>(part, threadIdx.x) : threadIdx.x);
@@ -242,6 +250,7 @@ __global__ void __launch_bounds__(NT, MINB) step3d_pull_slots_kernel(const __gri
     pdl_launch();
     if (!slots_item<LIST>(ka, Sp, tile, blockIdx.x / PARTS)) { pdl_wait(); return; }
     const Solve3 &S = *Sp;
+    if (LIST && noted_done(S)) { pdl_wait(); return; }
     const int part = blockIdx.x % PARTS;
     const unsigned tid = threadIdx.x;
     const unsigned P = (unsigned)S.plane, nf = (unsigned)S.nfluid;
@@ -325,6 +334,13 @@ __global__ void __launch_bounds__(NT, MINB) step3d_links_slots_kernel(const __gr
     const unsigned P = (unsigned)S0.plane, nf = (unsigned)S0.nfluid;
     const unsigned i0 = (unsigned)tile * (TPB * TILE_NPT) + (SPLIT ? split_voxel<NT, 1>(part, tid) : tid);
     const int ng = min(S0.group, MAX_GROUP);
+    if constexpr (LIST) {
+        bool done = true;
+#pragma unroll
+        for (int d = 0; d < MAX_GROUP; ++d)
+            if (d < ng) done = noted_done(Sp[d]) && done;
+        if (done) { pdl_wait(); return; }
+    }
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
         const unsigned i = i0 + j * TPB;

@@ -34,7 +34,7 @@ def _solid(n=64):
 
 
 RUN = [1e-6, 0.0, 0.0]
-STOP = [1e3, 0.0, 0.0]      # the flux is not finite by the first lag: the solve ends there
+STOP = [1e3, 0.0, 0.0]      # the flux is not finite within some hundred steps: the solve ends there
 
 
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
@@ -47,5 +47,35 @@ def test_directions(gpu, prec):
             solve3d(_solid(), forces, p)
         except LBMError as e:
             assert "non-finite" in str(e)
+
+    _check(_timed(lambda: go([RUN])), _timed(lambda: go([STOP] * 3 + [RUN])), _timed(lambda: go([RUN] * 4)))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16", "bf16"])
+def test_directions_that_end_apart(gpu, prec):
+    """Directions keep their bits when others of the call end before them."""
+    from flow_anizotropy_b200.solver import Params3D, solve3d
+    solid = (np.random.default_rng(3).random((20, 8, 5)) < 0.3).astype(np.uint8).repeat(2, 1).repeat(5, 2)
+    F = 1e-6 * np.array([[1, 0, 0], [0, 0, 1], [0, 1, 0], [1, -3, 0], [0, 2, 5]])
+    p = Params3D(eps=2e-3, lag=40, min_steps=80, max_steps=4000, avg_steps=150, precision=prec, criterion="drift")
+    together, _, _ = solve3d(solid, F, p)
+    assert len({r.steps for r in together}) > 2
+    for f, x in zip(F, together):
+        (y,), _, _ = solve3d(solid, [f], p)
+        assert (x.steps, x.converged) == (y.steps, y.converged)
+        assert np.array_equal(x.q, y.q) and np.array_equal(x.se, y.se)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16"])
+def test_batch_between_polls(gpu, prec):
+    from flow_anizotropy_b200.solver import Batch, Params3D
+    p = Params3D(eps=0.0, lag=64, min_steps=64, max_steps=64 * 40, avg_steps=0, precision=prec, criterion="drift")
+
+    def go(forces):
+        b = Batch(precision=prec, hbm_budget=2 ** 33, chunk=64)
+        assert b.submit(_solid(), forces, p, tag=0)
+        b.run(40)
+        assert len(b.poll()) == 1
+        b.close()
 
     _check(_timed(lambda: go([RUN])), _timed(lambda: go([STOP] * 3 + [RUN])), _timed(lambda: go([RUN] * 4)))
