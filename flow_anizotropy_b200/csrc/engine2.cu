@@ -68,20 +68,61 @@ static int run_plain2d(lbm_ctx *ctx, std::vector<Solve2> &hs, Solve2 *d_solves, 
                        std::vector<State2> &hst)
 {
     const int n = (int)hs.size();
-    long long s = 0, base = 0;        // steps done; s_base of every solve (host copy)
+    long long s = 0, base = 0;        // steps done; s_base of the unfinished solves (host copy)
     StepArgs2 a;
     a.solves = d_solves; a.step = 0; a.bit = -1;
     const int ntiles = hs[0].ntiles;
     bool masks = false;               // State2's step masks are those of s_base
+    // the first m records on the device are the unfinished solves, the only
+    // ones that are launched (a step requests its populations before it knows
+    // whether the solve runs); the others follow them, so that a chunk graph
+    // made for more solves stays right until it is made anew
+    int m = n;
+    bool stale = false;               // the graph launches solves that have finished
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     struct GraphGuard {
         cudaGraph_t &g; cudaGraphExec_t &e;
         ~GraphGuard() { if (e) cudaGraphExecDestroy(e); if (g) cudaGraphDestroy(g); }
     } guard{graph, exec};
+    auto capture = [&]() -> int {
+        if (graph) CK(cudaGraphDestroy(graph));
+        graph = nullptr;
+        CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+        cudaError_t e = cudaSuccess;
+        // launch i of a chunk runs step i + 1 after s_base (even)
+        for (int i = 0; i < CHUNK2 && e == cudaSuccess; ++i) {
+            StepArgs2 g = a;
+            g.step = i;
+            g.bit = i;
+            e = launch_step2d((i & 1) == 0, ntiles, m, ctx->stream, g);
+        }
+        if (e == cudaSuccess) e = launch_advance2d(d_solves, m, CHUNK2, ctx->stream);
+        const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
+        CK(e);
+        CK(e2);
+        if (exec) CK(cudaGraphExecDestroy(exec));     // a running one is freed when it has ended
+        exec = nullptr;
+        CK(cudaGraphInstantiate(&exec, graph, 0));
+        stale = false;
+        return LBM_OK;
+    };
     for (;;) {
         CK(cudaMemcpyAsync(hst.data(), d_states, sizeof(State2) * n, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
+        int live = 0;
+        for (int j = 0; j < n; ++j) live += hst[j].phase < PH_DONE;
+        if (live && live < m) {
+            std::vector<Solve2> order;
+            order.reserve(n);
+            for (int done = 0; done < 2; ++done)
+                for (int j = 0; j < n; ++j)
+                    if ((hst[j].phase >= PH_DONE) == (done != 0)) order.push_back(hs[j]);
+            CK(cudaMemcpyAsync(d_solves, order.data(), sizeof(Solve2) * n, cudaMemcpyHostToDevice, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
+            m = live;
+            stale = exec != nullptr;
+        }
         long long target = LLONG_MAX;
         for (int j = 0; j < n; ++j) {
             const State2 &st = hst[j];
@@ -96,36 +137,28 @@ static int run_plain2d(lbm_ctx *ctx, std::vector<Solve2> &hs, Solve2 *d_solves, 
         }
         if (target == LLONG_MAX) break;
         if (!exec && target - s >= CHUNK2) {
-            CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-            cudaError_t e = cudaSuccess;
-            // launch i of a chunk runs step i + 1 after s_base (even)
-            for (int i = 0; i < CHUNK2 && e == cudaSuccess; ++i) {
-                StepArgs2 g = a;
-                g.step = i;
-                g.bit = i;
-                e = launch_step2d((i & 1) == 0, ntiles, n, ctx->stream, g);
-            }
-            if (e == cudaSuccess) e = launch_advance2d(d_solves, n, CHUNK2, ctx->stream);
-            const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &graph);
-            CK(e);
-            CK(e2);
-            CK(cudaGraphInstantiate(&exec, graph, 0));
+            const int rc = capture();
+            if (rc) return rc;
         }
         while (s < target) {
             if (exec && (s & 1) == 0 && target - s >= CHUNK2) {
                 if (base != s || !masks) {
                     // a chunk numbers its steps from s_base: catch up with the
                     // single steps, and find the chunk's step flags
-                    CK(launch_advance2d(d_solves, n, s - base, ctx->stream));
+                    CK(launch_advance2d(d_solves, m, s - base, ctx->stream));
                     base = s;
                     masks = true;
                 }
                 CK(cudaGraphLaunch(exec, ctx->stream));
                 s += CHUNK2;
                 base += CHUNK2;
+                if (stale) {           // made anew while a chunk of the old one runs
+                    const int rc = capture();
+                    if (rc) return rc;
+                }
             } else {
                 a.step = s - base;
-                CK(launch_step2d((s & 1) == 0, ntiles, n, ctx->stream, a));
+                CK(launch_step2d((s & 1) == 0, ntiles, m, ctx->stream, a));
                 ++s;
             }
         }

@@ -184,9 +184,19 @@ extern "C" int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, i
     // direction's controller can change phase, then read the states back
     StepArgs2 a;
     a.solves = d_solves; a.bit = -1;
+    int m = ndir;                      // the first m records are the unfinished solves, the only ones launched
     for (long long s = 0;;) {
         CK(cudaMemcpyAsync(hst, d_states, sizeof(State2) * ndir, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        Solve2 live[kDirs];
+        int nlive = 0;
+        for (int j = 0; j < ndir; ++j)
+            if (hst[j].phase < PH_DONE) live[nlive++] = hs[j];
+        if (nlive && nlive < m) {
+            CK(cudaMemcpyAsync(d_solves, live, sizeof(Solve2) * nlive, cudaMemcpyHostToDevice, st));
+            CK(cudaStreamSynchronize(st));
+            m = nlive;
+        }
         long long target = LLONG_MAX;
         for (int j = 0; j < ndir; ++j) {
             const Ctl2 &c = hs[j].c;
@@ -201,7 +211,7 @@ extern "C" int lbm_solve2d_noalloc(lbm_ctx *ctx, const uint8_t *solid, int nx, i
         if (target == LLONG_MAX) break;
         for (; s < target; ++s) {
             a.step = s;
-            CK(launch_step2d((s & 1) == 0, hs[0].ntiles, ndir, st, a));
+            CK(launch_step2d((s & 1) == 0, hs[0].ntiles, m, st, a));
         }
     }
 

@@ -79,3 +79,58 @@ def test_batch_between_polls(gpu, prec):
         b.close()
 
     _check(_timed(lambda: go([RUN])), _timed(lambda: go([STOP] * 3 + [RUN])), _timed(lambda: go([RUN] * 4)))
+
+
+def test_images(gpu):
+    from flow_anizotropy_b200.solver import Params2D, solve2d_many
+    slow = np.ones((256, 256), np.uint8)
+    slow[28:228] = 0                                   # one wide channel along x
+    fast = np.zeros((256, 256), np.uint8)
+    fast[::8] = fast[1::8] = 1                         # channels of 6 rows
+    p = Params2D(eps=1e-3, lag=500, hold=2, min_steps=1000, max_steps=20000, avg_steps=500, avg_sample=50)
+
+    def go(images):
+        runs, _ = solve2d_many(np.stack(images), [[1e-6, 0.0]], p)
+        return runs
+
+    runs = go([slow] + [fast] * 31)
+    assert runs[0][0].steps == 20500 and all(r[0].steps < 4000 for r in runs[1:])
+    _check(_timed(lambda: go([slow])), _timed(lambda: go([slow] + [fast] * 31)), _timed(lambda: go([slow] * 32)))
+
+
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_images_that_end_apart(gpu, noalloc):
+    """Solves keep their bits when others of the call end before them."""
+    import ctypes as C
+
+    from flow_anizotropy_b200 import _lib, solver
+    from flow_anizotropy_b200.solver import Params2D, solve2d, solve2d_many
+    rng = np.random.default_rng(4)
+    images = (rng.random((5, 12, 40)) < np.array([0.0, 0.1, 0.2, 0.3, 0.4])[:, None, None]).astype(np.uint8).repeat(2, 2)
+    images[:, 0] = 1
+    p = Params2D(eps=1e-3, lag=150, hold=2, min_steps=300, max_steps=6000, avg_steps=250, avg_sample=50)
+    F = [[1e-6, 0.0], [0.0, 1e-6], [2e-6, 1e-6]][:2 if noalloc else 3]
+
+    def same(x, y):
+        # (the field residual's blocks add up in any order, then it is rounded to float)
+        return (x.steps, x.converged) == (y.steps, y.converged) and np.array_equal(x.q, y.q) and \
+            np.array_equal(x.se, y.se) and abs(x.fieldres - y.fieldres) <= 2.0 ** -22 * y.fieldres
+
+    alone = [[solve2d(im, [f], p)[0][0] for f in F] for im in images]
+    assert len({r.steps for row in alone for r in row}) > 2
+    if not noalloc:
+        together, _ = solve2d_many(images, F, p)
+    else:
+        together = []
+        for im in images:
+            ctx, c = _lib.context(0), p.to_c()
+            force = np.ascontiguousarray(F, np.float64)
+            res = (_lib.Result2D * len(F))()
+            rc = ctx.L.lbm_solve2d_noalloc(ctx.h, im.ctypes.data_as(C.POINTER(C.c_uint8)), im.shape[1], im.shape[0], len(F),
+                                           force.ctypes.data_as(C.POINTER(C.c_double)), C.byref(c), res, None)
+            ctx.check(rc, ok=(_lib.LBM_OK, _lib.LBM_NOT_CONVERGED))
+            together.append([solver.Result2D(q=np.array(r.q[:]), se=np.array(r.se[:]), steps=int(r.steps),
+                                             converged=int(r.converged), status=int(r.status), fieldres=float(r.fieldres))
+                             for r in res])
+    for row, ref in zip(together, alone):
+        assert all(same(x, y) for x, y in zip(row, ref))
