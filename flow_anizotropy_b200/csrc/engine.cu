@@ -539,6 +539,44 @@ static cudaError_t launch_plain_slots(const std::vector<Solve3> &hs, int j0, int
     return e;
 }
 
+// Step launches of one call's solves (run_plain3d and the autotuner).
+struct PlainSteps {
+    int prec, variant;                // the effective variant
+    bool w1;
+    StepArgs a, ae;                   // work lists: (solve, tile) items, and the even steps' (grouped variants')
+    cudaStream_t stream;
+    bool slots, gall;
+    std::vector<Solve3> live;         // slots variants: the records to step, their groups set
+
+    PlainSteps(int prec_, int variant_, bool w1_, const StepArgs &a_, const StepArgs &ae_, cudaStream_t s)
+        : prec(prec_), variant(variant_), w1(w1_), a(a_), ae(ae_), stream(s),
+          slots(lbm_slots_variant(prec_, variant_)), gall(lbm_grouped_all(prec_, variant_)) {}
+
+    // `count` steps from relative step rel on (the step after s0 steps done, bit
+    // `bit` of the masks): every group of directions in turn takes all of
+    // them, so that its lattices stay in L2 from step to step
+    cudaError_t launch(long long rel, long long s0, int bit, int count) const
+    {
+        cudaError_t e = cudaSuccess;
+        const int m = slots ? (int)live.size() : 1;
+        const int group = slots ? plain_group(prec, variant, live[0], m) : 1;
+        for (int j = 0; j < m && e == cudaSuccess; j += group)
+            for (int i = 0; i < count && e == cudaSuccess; ++i) {
+                const int n4 = (int)((s0 + i + 1) & 3);
+                const bool odd = n4 & 1;
+                StepArgs x = (slots || (odd && !gall)) ? a : ae;
+                x.step = rel + i;
+                if (slots) {
+                    x.bit = bit + i; x.n4 = n4;
+                    e = launch_plain_slots(live, j, std::min(group, m - j), prec, variant, w1, x, stream);
+                } else {
+                    e = lbm_launch_step(prec, variant, w1, odd, dim3(x.nwork), stream, x);
+                }
+            }
+        return e;
+    }
+};
+
 static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, State3 *d_states,
                        const int2 *d_work, int nwork, int prec, int variant, std::vector<State3> &hst)
 {
@@ -577,43 +615,18 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
     a.starve = ctx->test_starve;
     ae.wait_ns = a.wait_ns;
     ae.starve = a.starve;
-    const bool gall = lbm_grouped_all(prec, variant);
-    const bool slots = lbm_slots_variant(prec, variant);
-    // slots variants: the records of the unfinished solves, the only ones that
-    // are launched.  (Their kernels request populations before they know
-    // whether the solve runs, so a finished one would go on reading its
-    // lattice: one direction of 64^3 at porosity 0.8 beside three that had
-    // finished took 19.2 us per step in FP64 and 11.7 in FP32, now 12.2 and
-    // 6.5; alone 10.7 and 5.4.)
-    std::vector<Solve3> live;
+    PlainSteps steps(prec, variant, w1, a, ae, ctx->stream);
+    // slots variants launch the records of the unfinished solves only.  (Their
+    // kernels request populations before they know whether the solve runs, so a
+    // finished one would go on reading its lattice: one direction of 64^3 at
+    // porosity 0.8 beside three that had finished took 19.2 us per step in FP64
+    // and 11.7 in FP32, now 12.2 and 6.5; alone 10.7 and 5.4.)
     auto relist = [&] {
-        live.clear();
+        steps.live.clear();
         for (int j = 0; j < n; ++j)
-            if (hst[j].phase < PH_DONE) live.push_back(hs[j]);
-        const int m = (int)live.size();
-        for (int j = 0; j < m; ++j) live[j].group = j % MAX_GROUP ? 0 : std::min(MAX_GROUP, m - j);
-    };
-    // `count` steps from relative step rel on (the step after s0 steps done, bit
-    // `bit` of the masks): every group of directions in turn takes all of
-    // them, so that its lattices stay in L2 from step to step
-    auto launch = [&](long long rel, long long s0, int bit, int count) {
-        cudaError_t e = cudaSuccess;
-        const int m = slots ? (int)live.size() : 1;
-        const int group = slots ? plain_group(prec, variant, live[0], m) : 1;
-        for (int j = 0; j < m && e == cudaSuccess; j += group)
-            for (int i = 0; i < count && e == cudaSuccess; ++i) {
-                const int n4 = (int)((s0 + i + 1) & 3);
-                const bool odd = n4 & 1;
-                StepArgs x = (slots || (odd && !gall)) ? a : ae;
-                x.step = rel + i;
-                if (slots) {
-                    x.bit = bit + i; x.n4 = n4;
-                    e = launch_plain_slots(live, j, std::min(group, m - j), prec, variant, w1, x, ctx->stream);
-                } else {
-                    e = lbm_launch_step(prec, variant, w1, odd, dim3(x.nwork), ctx->stream, x);
-                }
-            }
-        return e;
+            if (hst[j].phase < PH_DONE) steps.live.push_back(hs[j]);
+        const int m = (int)steps.live.size();
+        for (int j = 0; j < m; ++j) steps.live[j].group = j % MAX_GROUP ? 0 : std::min(MAX_GROUP, m - j);
     };
     // reduce and control the deferred single launches (before s_base moves,
     // before a chunk reuses their slots, and before the states are read)
@@ -631,7 +644,7 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
         graph = nullptr;
         CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         // launch i of a chunk runs step i + 1 after s_base (a multiple of 4)
-        cudaError_t e = launch(0, 0, 0, kGraphSteps3);
+        cudaError_t e = steps.launch(0, 0, 0, kGraphSteps3);
         if (e == cudaSuccess && defer) e = launch_deferred3d(d_solves, n, 0, kGraphSteps3, qb, 1, kGraphSteps3, ctx->stream);
         if (e == cudaSuccess && !defer) {
             advance3d_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(d_solves, n, kGraphSteps3);
@@ -647,9 +660,9 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
     for (;;) {
         CK(cudaMemcpyAsync(hst.data(), d_states, sizeof(State3) * n, cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        const size_t had = live.size();
+        const size_t had = steps.live.size();
         relist();
-        stale = stale || (slots && exec && live.size() != had);
+        stale = stale || (steps.slots && exec && steps.live.size() != had);
         long long target = LLONG_MAX;
         for (int j = 0; j < n; ++j) {
             const State3 &st = hst[j];
@@ -692,7 +705,7 @@ static int run_plain3d(lbm_ctx *ctx, std::vector<Solve3> &hs, Solve3 *d_solves, 
                            !(exec && ((s + count) & 3) == 0 && target - s - count >= kGraphSteps3)) ++count;
                     if (!pending) pend0 = s - base;
                 }
-                CK(launch(s - base, s, pending, count));
+                CK(steps.launch(s - base, s, pending, count));
                 s += count;
                 if (defer && (pending += count) == DEFER_SLOTS) CK(flush());
             }
@@ -891,8 +904,8 @@ extern "C" int lbm_variant_count(int precision)
 }
 
 // Autotuner: every variant runs the same fixed number of steps on the same
-// resident lattices (directions as a batch, like a tensor solve), timed with
-// CUDA events on the launch stream.
+// resident lattices with the launches of a tensor solve, timed with CUDA
+// events on the launch stream.
 extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, int nz, int ndir,
                           int precision, int nsteps, double *ms_per_step, int *best)
 {
@@ -976,9 +989,10 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
         a.work = static_cast<const int2 *>(w.p);
         a.nwork_dev = nullptr;
         a.nwork = (int)work.size();
-        if (lbm_defers(precision)) { a.defer = 1; a.bit = 0; }      // no step reduces (redm = 0)
+        // no step reduces (no lag multiple comes, redm = 0): the partials, of
+        // one slot of whole tiles per direction, are never written
+        if (lbm_defers(precision)) { a.defer = 1; a.bit = 0; }
         const int ev = lbm_effective_variant(precision, v, proto.meta != nullptr);
-        const bool slots = lbm_slots_variant(precision, ev);
         StepArgs ae = a;
         DevMem gw(ctx->stream);
         if (lbm_grouped_variant(precision, ev)) {
@@ -990,21 +1004,22 @@ extern "C" int lbm_tune3d(lbm_ctx *ctx, const uint8_t *solid, int nx, int ny, in
             ae.work = static_cast<const int2 *>(gw.p);
             ae.nwork = (int)items.size();
         }
-        const bool gall = lbm_grouped_all(precision, ev);
-        auto launch = [&](long long s) {
-            const bool odd = ((s + 1) & 1) == 1;
-            StepArgs &x = (odd && !gall) ? a : ae;
-            x.step = s;
-            if (slots) {
-                x.n4 = (int)((s + 1) & 3);
-                return launch_plain_slots(hs, 0, ndir, precision, ev, true, x, ctx->stream);
-            }
-            return lbm_launch_step(precision, ev, true, odd, dim3(x.nwork), ctx->stream, x);
-        };
+        // the launches of a solve: directions in groups, a pass of steps at a time
+        PlainSteps steps(precision, ev, true, a, ae, ctx->stream);
+        steps.live = hs;
         long long s = 0;
-        for (int i = 0; i < std::max(2, nsteps / 4); ++i) CK(launch(s++));
+        auto run = [&](int count) -> cudaError_t {
+            cudaError_t e = cudaSuccess;
+            for (int i = 0; i < count && e == cudaSuccess; i += DEFER_SLOTS) {
+                const int c = std::min(DEFER_SLOTS, count - i);
+                e = steps.launch(s, s, 0, c);
+                s += c;
+            }
+            return e;
+        };
+        CK(run(std::max(2, nsteps / 4)));
         CK(cudaEventRecord(e0, ctx->stream));
-        for (int i = 0; i < nsteps; ++i) CK(launch(s++));
+        CK(run(nsteps));
         CK(cudaEventRecord(e1, ctx->stream));
         CK(cudaEventSynchronize(e1));
         float ms = 0.f;
