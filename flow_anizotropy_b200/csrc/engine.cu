@@ -509,6 +509,9 @@ static bool plain_split(int prec, int variant, const Solve3 &S, int ndir)
 // well as one does, but not 96 (FP64 72^3 with 100 MB allowed: 36.6).  The
 // 16-bit even step shares a voxel's link slots between the directions and is
 // not bound by DRAM (51 GLUPS in and out of L2), so it keeps them together.
+// An uneven split costs little: four FP64 directions of 64^3 (23 MB each) take
+// 30.4 us as 3 + 1, 29.7 as 2 + 2, 33.4 all together and 34.7 one at a time;
+// of 56^3 (19 MB) 25.4 all together, 25.2 as 3 + 1, 25.0 as 2 + 2.
 constexpr long long L2_GROUP_BYTES = 80ll << 20, L2_ONE_BYTES = 88ll << 20, L2_ONE_BYTES_PULL = 112ll << 20;
 static int plain_group(int prec, int variant, const Solve3 &S, int ndir)
 {
