@@ -54,8 +54,11 @@ struct Phys3 : PhysF {
 // twice with the exact remainder (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990: with y correctly
 // rounded and q within one unit in the last place, q + (a - b q) y rounds to
-// a / b; the first correction makes q that good).  Needs no subnormal
-// remainders, which quotients of populations and relaxation times never have.
+// a / b; the first correction makes q that good).  The remainders must not be
+// subnormal: not so for |a| below 2^-969, as from a body force under 1e-291,
+// which moves no population (those are multiples of 2^-57), where the last bit
+// of the velocity may differ.  An infinite or zero b gives NaN where the
+// division gives an infinity; the solve's flux is not finite either way.
 // Five multiply-adds and no branch, where one divisor serves many quotients.
 __device__ __forceinline__ double div_by(double a, double b, double y)
 {
@@ -73,9 +76,9 @@ __device__ __forceinline__ double div_by(double a, double b, double y)
 // quotients by the density share one reciprocal, and the 19 by tau use its
 // host-rounded reciprocal (div_by), or are left out for tau = 1 (W1,
 // x / 1 == x).  22 divisions and some 330 other operations per voxel became
-// one reciprocal, 15 multiply-adds and some 330 operations: per step of the
-// three directions, 64^3 at porosity 0.60: 41.7 -> 28.2 us, 80^3 at 0.75:
-// 97.1 -> 74.0 us, one direction of 32^3: 10.3 -> 7.5 us.
+// one reciprocal, 15 multiply-adds (110 for tau != 1) and some 330 operations:
+// per step of the three directions at tau = 1, 64^3 at porosity 0.60: 41.7 ->
+// 28.2 us, 80^3 at 0.75: 97.1 -> 74.0 us, one direction of 32^3: 10.3 -> 7.5 us.
 // g holds the pre-collision values on entry and the post-collision ones on exit.
 // ---------------------------------------------------------------------------
 template <bool W1>

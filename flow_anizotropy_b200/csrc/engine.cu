@@ -488,7 +488,7 @@ bool lbm_slots_variant(int prec, int variant)
 // part of a step.  The pull form's whole tiles pack better (its split tiles
 // measured the same at 96^3, 42.5 against 42.6 us per step), so it splits
 // only where whole tiles do not fill the SMs' block slots once.
-constexpr int SPLIT_MAX_TILES = 8192, SPLIT_MAX_TILES_PULL = 444;
+constexpr int SPLIT_MAX_TILES = 8192, SPLIT_MAX_TILES_PULL = 3 * 148;   // 3 blocks per SM
 static bool plain_split(int prec, int variant, const Solve3 &S, int ndir)
 {
     variant = lbm_effective_variant(prec, variant, S.meta != nullptr);

@@ -245,7 +245,8 @@ __device__ __forceinline__ void finish_tile2(const Solve2 &S, int tile, long lon
     }
 }
 
-// a / b per lane, correctly rounded, from y = RN(1/b) (see div_by).
+// a / b per lane, correctly rounded, from y = RN(1/b) (see div_by; here for
+// |a| from 2^-102 on, 2e-31).
 __device__ __forceinline__ float2 div_by2(float2 a, float2 b, float2 y)
 {
     const float2 nb = F32x2::neg(b);

@@ -22,7 +22,9 @@
 //             final entry = pore count): the rank of voxel x in row r is
 //             wpre[r*wpr + x/32] + popc(~mask word & bits below x).
 //   fnode     linear index of each pore voxel (neighbour steps need x, y, z).
-//   partials  one double3 per tile, written only on reduction steps.
+//   partials  one double3 per tile (of a split tile one per warp), times
+//             DEFER_SLOTS where the reduction is deferred; written only on
+//             reduction steps.
 //
 // Work is a list of (solve, tile) items; a tile is TPB*NPT consecutive pore
 // voxels of one lattice.  One launch advances every listed solve by one step,
@@ -130,7 +132,7 @@ struct Solve3 {
     float scale, inv_scale;
     Phys3 P;
     Ctl3 c;
-    double *partials;     // ntiles * 3
+    double *partials;     // ntiles * 3, times DEFER_SLOTS if deferred, times TPB / 32 if split (lbm_partial_doubles)
     State3 *st;
     MDGeom md;            // dense moment form only
     int group;            // grouped even step: directions in the group led by this record (else 0)
